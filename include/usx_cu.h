@@ -152,7 +152,10 @@ int usx_cu_bf_plan_set_precision(usx_bf_plan* plan, int precision);
  * variant (plus a warm-up) `repeats` times, keeps the fastest in the plan,
  * writes every variant's mean milliseconds to ms_out[variant] (host, may be
  * NULL; usx_cu_bf_variant_count() entries), leaves the frame of the chosen
- * variant in `frame` and synchronises. Variant 0 is the default. */
+ * variant in `frame` and synchronises. A plan whose variant was neither set
+ * nor tuned reports 0; its IQ frames (coherent or select) take the
+ * channel-warp shape that a rule on pixels and events picks, its others
+ * variant 0. */
 int usx_cu_bf_variant_count(void);
 int usx_cu_bf_variant_info(int index, int* channel_group, int* tile_lines, int* min_blocks, int* warp_lines);
 /* The order in which variant i dispatches its CTA tiles: *deep_first = 1 when
@@ -168,9 +171,11 @@ int usx_cu_bf_variant_order(int index, int* deep_first);
  * warp (bulk copies on mbarriers, no CTA-wide barrier in the loop), 4
  * channel warps beside the pixel warps with the transmit terms tabulated per
  * pixel and event (the minimum-variance export, and the sums with the
- * channel combine in shared memory, in ascending channel order).
+ * channel combine in shared memory, in ascending channel order;
+ * tile_lines is the CTA's pixel warps, 32 x tile_lines pixels).
  * Families 1-4 fall back to variant 0 where they do not apply (RF data,
- * incoherent compounding; families 1 and 3 also need plane waves, family 2
+ * incoherent compounding, and for family 4 traces of one sample or of more
+ * than 2^23; families 1 and 3 also need plane waves, family 2
  * at most 256 channels). */
 int usx_cu_bf_variant_kind(int index, int* kind);
 int usx_cu_bf_plan_set_variant(usx_bf_plan* plan, int index);

@@ -58,6 +58,7 @@ struct BfArgs {
   int mv_subarray, mv_range_average;
   float mv_loading;
   int* status;           // context status word (set when a bounded wait gives up)
+  int tab_events;        // channel-warp kernels: events per transmit table
 };
 
 __device__ __forceinline__ float elem_x(const BfArgs& a, int ch) {
@@ -448,71 +449,82 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_fast_kernel(const B
 }
 
 // ------------------------------------------------------------------------
-// das_export_kernel: the minimum-variance export (compounded channel samples
-// y[frame][pixel][channel]) with the transmit side tabulated per pixel. A
-// CTA is kPW pixel warps x kCQ channel warps: the tile is kPW x 32 pixels
-// (das_fast_kernel's tile: kPW lines x 32 depths, warps of kWL lines x 32 /
-// kWL depths), and channel warp cq takes channels cq, cq + kCQ, ... in groups
-// of kG, so the kPW pixel warps that share a channel read the same trace
-// windows through L1. Per pass (one group of kG channels per channel warp)
-// the events go in chunks of kExpEv: the CTA first tabulates (transmit delay,
-// weighted transmit phasor, illumination weight) for its pixels and the
-// chunk's events, each thread for its own pixel, then every thread runs its
-// kG channels over the chunk. The transmit side is evaluated once per pixel,
-// event and pass instead of once per channel group; the per-channel sums are
-// das_fast_kernel's expressions in the same order, so the exported samples
-// are the same bit for bit.
-// das_csum_kernel is the same body for the plain sums (delay-and-sum, DMAS,
-// coherence factor): after each pass the channel warps stage their channel
-// values in the table's shared memory and channel warp 0's thread of each
-// pixel combines the pass's channels in ascending order, exactly as
-// das_fast_kernel's channel loop, so its frames are the same bit for bit;
-// the combine state lives in shared memory between passes. At 128 channels,
-// 75 plane waves, 512 x 1024: 4.20 ms per frame against 4.97 for
-// das_fast_kernel's best shape (three CTAs per SM; two, at 64 registers,
-// measured 5.6). Warps of 2 or 1 lines (x 16 or 32 depths) instead of 4:
-// 4.26 and 4.34 ms; 2 pixel warps x 8 channel warps (32 channels per pass,
-// half the passes and tables, half the pixel warps sharing a trace): 4.43.
-// Measured on the learned frame (128 ch, 75 plane waves, 512 x 1024): export
-// 4.83 ms with (kG, kPW, kCQ, kWL) = (4, 4, 4, 4) against 5.08 for
-// das_fast_kernel's best shape; (8, 4, 4, 4) 5.1, (8, 4, 4, 1) 5.6,
-// (8, 4, 2, 4) 5.3. The gathers' latency, not the transmit terms, bounds it.
-// Skipping the passes outside every pixel's aperture: 4.83 -> 4.38 ms; the
-// deepest tiles first: 4.38 -> 4.13 ms; chunks of 32 events instead of 16
-// (half the table barriers, the table in 64 KB of dynamic shared memory):
-// 4.13 -> 4.10 ms, and 4.21 -> 4.18 ms for das_csum_kernel.
-constexpr int kExpEv = 32;
-// Dynamic shared memory of the channel-warp kernels (the transmit table).
-__host__ __device__ constexpr size_t exp_table_bytes(int pixel_warps) {
-  return sizeof(float4) * kExpEv * 32 * pixel_warps;
+// The channel-warp kernels: das_export_kernel, the minimum-variance export
+// (compounded channel samples y[frame][pixel][channel]), and das_csum_kernel,
+// the plain sums (delay-and-sum, DMAS, coherence factor). A CTA is kPW pixel
+// warps x kCQ channel warps over a tile of kTL lines x 32 kPW / kTL depths
+// (warps of kWL lines x 32 / kWL depths). The transmit side (delay, weighted
+// phasor) is tabulated once per pixel and event in shared memory; then channel
+// warp cq takes channel group g0 + cq of kG channels per pass, over the groups
+// that reach any pixel of the tile. The pixel warps that share a channel read
+// the same trace windows through L1. Per-channel sums are das_fast_kernel's
+// expressions in the same order; das_csum_kernel stages a pass's channel
+// values in shared memory and combines them in ascending channel order, so
+// the samples and the frames are the same bit for bit.
+//
+// What bounds it: the gathers (two 8-byte loads per pixel, channel and event:
+// L1 hit rate 50%, 42% of the L1 data pipe, 56% issue at 32 warps per SM).
+// Per frame at 128 channels, 75 plane waves, 512 x 1024 pixels:
+//   4.18 ms  the table refilled in 32-event chunks on every pass of 16
+//            channels, one channel's loads waited for before the next's
+//   3.68 ms  the kG channels' loads all issued before the first is used
+//            (predicated by the index test, no branch per channel), floor by
+//            a directed-rounding addition instead of conversions, 64
+//            registers and two CTAs per SM instead of 40 and three
+//   2.87 ms  the table filled once per tile (up to kTabEvents events), passes
+//            over the tile's active channel groups alone, 32 channels a pass
+//   2.58 ms  index and interpolation arithmetic on FP32 pairs, tiles of 4
+//            lines x 8 depths (narrower trace windows: 3.6 -> 2.2 L1
+//            wavefronts per load)
+// Shapes (kG, kPW, kCQ, kWL, kTL) at 75 / 11 events, 512 x 1024 / 256 x 640:
+// (4,1,8,4,4) 2.58 / 0.253 ms, (4,2,8,4,8) 2.62 / 0.234, (4,2,4,4,8) 2.80 /
+// 0.219, (4,4,4,4,4) 4.02 / 0.208 (its 75-event table leaves one CTA per SM),
+// (4,2,8,2,2) 2.82 / 0.236, (2,2,8,4,8) 2.74 / 0.225, 8 channels per group
+// 4.5 / 0.319, 40 registers with three CTAs 3.5 / 0.226.
+constexpr int kTabEvents = 80;   // events a CTA tabulates at once (more go in chunks)
+
+// Dynamic shared memory of the channel-warp kernels: the transmit table of
+// `events` events and, for the sums, a pass's channel values, the channel
+// warps' aperture masks and the combine state, per pixel of the tile.
+__host__ __device__ constexpr size_t exp_smem_bytes(int events, int pixel_warps, int channel_warps, int group, bool sum) {
+  return static_cast<size_t>(32 * pixel_warps) *
+         (3 * sizeof(float) * events + (sum ? sizeof(float2) * channel_warps * group + 4 * channel_warps + 4 * 10 : 0));
 }
 
-template <int kG, int kPW, int kCQ, int kWL, bool kSum>
+// Sample indices take floor(idx) by one directed-rounding addition: 2^23 + idx
+// rounded down is 2^23 + floor(idx) for 0 <= idx < 2^23, its low mantissa bits
+// the integer (no conversion instruction, which run at a fraction of the FP32
+// rate). A negative, infinite or NaN index, or one of 2^23 and above, gives at
+// least 2^23: past every trace these kernels take.
+constexpr int kMaxFastSamples = 1 << 23;
+
+template <int kG, int kPW, int kCQ, int kWL, int kTL, bool kSum>
 __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long frame) {
-  static_assert(32 % kWL == 0 && kPW % kWL == 0, "warp shape must tile the CTA");
-  static_assert(sizeof(float2) * kCQ * kG <= sizeof(float4) * kExpEv, "a pass's channel values fit the table");
+  constexpr int kTD = 32 * kPW / kTL, kWD = 32 / kWL, kWarpCols = kTD / kWD;
+  static_assert(32 % kWL == 0 && kTL % kWL == 0 && kTD % kWD == 0 && kG % 2 == 0, "warp shape must tile the CTA");
+  constexpr int kPx = 32 * kPW;
   extern __shared__ float4 das_exp_smem[];
-  float4 (*tab)[32 * kPW] = reinterpret_cast<float4 (*)[32 * kPW]>(das_exp_smem);   // [kExpEv][pixel slot]
-  // kSum: a pass's channel values [channel of the pass][pixel slot] in the
-  // table's space once the pass's events are done, and each channel warp's
-  // aperture mask per pixel.
-  __shared__ unsigned act_s[kSum ? kCQ : 1][32 * kPW];
-  // kSum: each pixel's combine state (das, s, q, coh, incs, n_active), kept
-  // in shared memory rather than in registers through the event loops.
-  __shared__ float cs[kSum ? 10 : 1][32 * kPW];
-  float2* ys = reinterpret_cast<float2*>(das_exp_smem);
-  constexpr int kWD = 32 / kWL;
+  // [event of the chunk][pixel slot]: weighted transmit phasor, transmit delay.
+  float2* tab_w = reinterpret_cast<float2*>(das_exp_smem);
+  float* tab_t = reinterpret_cast<float*>(tab_w + a.tab_events * kPx);
+  // kSum: a pass's channel values [channel of the pass][pixel slot], each
+  // channel warp's aperture mask per pixel, and each pixel's combine state
+  // (das, s, q, coh, incs, n_active).
+  float2* ys = reinterpret_cast<float2*>(tab_t + a.tab_events * kPx);
+  unsigned* act_s = reinterpret_cast<unsigned*>(ys + (kSum ? kCQ * kG * kPx : 0));
+  float* cs = reinterpret_cast<float*>(act_s + (kSum ? kCQ * kPx : 0));
+  __shared__ int s_range[2];
   const int n0 = a.n_pix / a.n1;
-  const int tiles_depth = (a.n1 + 31) / 32;
+  const int tiles_depth = (a.n1 + kTD - 1) / kTD;
   const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
   const int pw = w % kPW, cq = w / kPW;
   const int pl = pw * 32 + ln;   // pixel slot in the tile
   // Deepest depth tiles first: the aperture, and with it a tile's active
   // passes, grows with depth, so the last CTAs of the grid are the lightest.
-  const int n_line_tiles = (n0 + kPW - 1) / kPW;
+  const int n_line_tiles = (n0 + kTL - 1) / kTL;
   const int line_tile = tile % n_line_tiles, depth_tile = tiles_depth - 1 - tile / n_line_tiles;
-  const int line = line_tile * kPW + (pw / kWL) * kWL + ln / kWD;
-  const int depth = depth_tile * 32 + (pw % kWL) * kWD + ln % kWD;
+  const int line = line_tile * kTL + (pw / kWarpCols) * kWL + ln / kWD;
+  const int depth = depth_tile * kTD + (pw % kWarpCols) * kWD + ln % kWD;
   const bool valid = line < n0 && depth < a.n1;
   const int pix = valid ? line * a.n1 + depth : 0;
   const float px = __ldg(a.points + 3 * pix), py = __ldg(a.points + 3 * pix + 1), pz = __ldg(a.points + 3 * pix + 2);
@@ -539,87 +551,141 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
   }
   const float2* iq = a.iq + frame * a.data_stride;
   const unsigned n_last = static_cast<unsigned>(a.n_smp - 1);
+  const long ev_stride = static_cast<long>(a.n_ch) * a.n_smp;
   const int n_groups = (a.n_ch + kG - 1) / kG;
-  const int n_pass = (n_groups + kCQ - 1) / kCQ;
-  // kSum: the channel combine of das_fast_tile, run by channel warp 0's
-  // thread of each pixel over the channels in ascending order.
+  const float2 neg_t0 = make_float2(-a.t0, -a.t0), fs2 = make_float2(a.fs, a.fs);
+  const float2 kBig2 = make_float2(8388608.0f, 8388608.0f), kMinus2 = make_float2(-1.0f, -1.0f);
+
+  // The channel groups any pixel of the tile can use: the aperture interval
+  // |x_e - x_p| <= z / (2 F#) outside which every window is zero, widened by
+  // two channels for rounding. The passes run over these groups alone.
+  if (threadIdx.x == 0) {
+    s_range[0] = a.n_ch;
+    s_range[1] = -1;
+  }
+  __syncthreads();   // (also: the previous tile's shared memory is no longer read)
+  if (cq == 0) {
+    int c_lo = a.n_ch, c_hi = -1;
+    if (valid && pz > 0.0f) {
+      const float half = 0.5f * pz / fmaxf(a.f_number, 1e-3f), top = static_cast<float>(a.n_ch - 1);
+      c_lo = static_cast<int>(fminf(fmaxf(floorf((px - half) / a.pitch + a.half_nm1) - 2.0f, 0.0f), top));
+      c_hi = static_cast<int>(fminf(fmaxf(ceilf((px + half) / a.pitch + a.half_nm1) + 2.0f, 0.0f), top));
+    }
+    c_lo = __reduce_min_sync(0xffffffffu, c_lo);
+    c_hi = __reduce_max_sync(0xffffffffu, c_hi);
+    if (ln == 0) {
+      atomicMin(&s_range[0], c_lo);
+      atomicMax(&s_range[1], c_hi);
+    }
+  }
   if (kSum && cq == 0)
 #pragma unroll
-    for (int i = 0; i < 10; ++i) cs[i][pl] = 0.0f;
-  for (int pass = 0; pass < n_pass; ++pass) {
-    const int grp = pass * kCQ + cq;
-    const int g = grp * kG;
-    float rt[kG];
+    for (int i = 0; i < 10; ++i) cs[i * kPx + pl] = 0.0f;
+  __syncthreads();
+  const int g_lo = s_range[1] < s_range[0] ? 0 : s_range[0] / kG;
+  const int g_hi = s_range[1] < s_range[0] ? 0 : s_range[1] / kG + 1;
+  if (!kSum && valid)
+    for (int grp = cq; grp < n_groups; grp += kCQ) {   // the groups no pass visits
+      if (grp >= g_lo && grp < g_hi) continue;
+      for (int ch = grp * kG; ch < min(a.n_ch, grp * kG + kG); ++ch)
+        a.y_out[(frame * a.n_pix + pix) * a.n_ch + ch] = make_float2(0.f, 0.f);
+    }
+
+  const bool one_chunk = ev_hi - ev_lo <= a.tab_events;
+  for (int g0 = g_lo; g0 < g_hi; g0 += kCQ) {
+    const int grp = g0 + cq, g = grp * kG;
+    float2 rt[kG / 2];   // receive delays, two channels a pair
     unsigned mask = 0u;
 #pragma unroll
     for (int k = 0; k < kG; ++k) {
       const int ch = g + k;
-      rt[k] = 0.0f;
-      if (valid && ch < a.n_ch) {
+      float r = INFINITY;   // an inactive channel's sample index is past every trace
+      if (valid && grp < g_hi && ch < a.n_ch) {
         const float ex = elem_x(a, ch);
         if (aperture_weight(ex, px, pz, a.f_number, a.rx_window, a.tukey_alpha) > 0.0f) {
           mask |= 1u << k;
-          rt[k] = dist3(ex, 0.0f, 0.0f, px, py, pz) / a.c;
+          r = dist3(ex, 0.0f, 0.0f, px, py, pz) / a.c;
         }
       }
+      if (k & 1)
+        rt[k / 2].y = r;
+      else
+        rt[k / 2].x = r;
     }
-    float ar[kG], ai[kG];
+    float2 acc[kG];
 #pragma unroll
-    for (int k = 0; k < kG; ++k) ar[k] = ai[k] = 0.0f;
-    // A pass whose kCQ x kG channels are outside every pixel's aperture (the
-    // shallow tiles') skips the transmit table and the events; its samples
-    // are written as zeros below.
-    const int c_end = __syncthreads_or(mask != 0u) ? ev_hi : ev_lo;
-    for (int c0 = ev_lo; c0 < c_end; c0 += kExpEv) {
-      const int c1 = min(c_end, c0 + kExpEv);
-      // The chunk's table: (tau, tw cos, tw sin, tw) for this thread's pixel.
-      __syncthreads();
-      for (int e = c0 + cq; e < c1; e += kCQ) {
-        const TxDev& t = a.tx[e];
-        float tw;
-        if (!valid)
-          tw = 0.0f;
-        else if (select)
-          tw = (best_ev == e && best_w > 0.0f) ? 1.0f : 0.0f;
-        else if (a.tx_weighting)
-          tw = tx_sensitivity_fast(t, px, pz, a.lambda);
-        else
-          tw = 1.0f;
-        float4 ent = make_float4(0.f, 0.f, 0.f, tw);
-        if (tw > 0.0f) {
-          const float tau = tx_arrival(t, px, py, pz, a.c);
-          float tc = 1.0f, ts = 0.0f;
-          if (a.fdem > 0.0f) sincosf(a.two_pi_f * tau, &ts, &tc);
-          ent = make_float4(tau, tw * tc, tw * ts, tw);
+    for (int k = 0; k < kG; ++k) acc[k] = make_float2(0.f, 0.f);
+    for (int c0 = ev_lo; c0 < ev_hi; c0 += a.tab_events) {
+      const int c1 = min(ev_hi, c0 + a.tab_events);
+      if (!one_chunk || g0 == g_lo) {
+        // The chunk's table: (tw cos, tw sin) and tau for this thread's
+        // pixel; +inf where the event does not reach it (or its delay is
+        // infinite), which puts every sample index past the trace.
+        if (!one_chunk) __syncthreads();
+        for (int e = c0 + cq; e < c1; e += kCQ) {
+          const TxDev& t = a.tx[e];
+          float tw;
+          if (!valid)
+            tw = 0.0f;
+          else if (select)
+            tw = (best_ev == e && best_w > 0.0f) ? 1.0f : 0.0f;
+          else if (a.tx_weighting)
+            tw = tx_sensitivity_fast(t, px, pz, a.lambda);
+          else
+            tw = 1.0f;
+          float tau = INFINITY;
+          float2 ph = make_float2(0.f, 0.f);
+          if (tw > 0.0f) {
+            tau = tx_arrival(t, px, py, pz, a.c);
+            float tc = 1.0f, ts = 0.0f;
+            if (a.fdem > 0.0f) sincosf(a.two_pi_f * tau, &ts, &tc);
+            if (!isinf(tau)) ph = make_float2(tw * tc, tw * ts);
+          }
+          tab_w[(e - c0) * kPx + pl] = ph;
+          tab_t[(e - c0) * kPx + pl] = tau;
         }
-        tab[e - c0][pl] = ent;
+        __syncthreads();
       }
-      __syncthreads();
       if (!mask) continue;
-      for (int e = c0; e < c1; ++e) {
-        const float4 ent = tab[e - c0][pl];
-        if (ent.w <= 0.0f) continue;
-        const float tau = ent.x, wr = ent.y, wi = ent.z;
-        const float2* trace = iq + (static_cast<long>(e) * a.n_ch + g) * a.n_smp;
+      const float2* trace = iq + c0 * ev_stride + static_cast<long>(g) * a.n_smp;
+      const int n_ev = c1 - c0;
+#pragma unroll 1
+      for (int e = 0; e < n_ev; ++e, trace += ev_stride) {
+        const float tau = tab_t[e * kPx + pl];
+        if (isinf(tau)) continue;
+        const float2 w2 = tab_w[e * kPx + pl];
+        const float2 tau2 = make_float2(tau, tau), wr2 = make_float2(w2.x, w2.x);
+        // Every load of the group is issued before the first is used; an
+        // index outside the trace (an inactive channel's too, which may be
+        // past the last) loads the group's first pair and adds nothing.
+        float2 s0[kG], s1[kG], f2[kG / 2];
+        bool in[kG];
+#pragma unroll
+        for (int q = 0; q < kG / 2; ++q) {
+          const float2 idx = __fmul2_rn(__fadd2_rn(__fadd2_rn(tau2, rt[q]), neg_t0), fs2);
+          const float2 t = __fadd2_rd(idx, kBig2);
+          f2[q] = __fadd2_rn(idx, __ffma2_rn(t, kMinus2, kBig2));   // idx - floor(idx)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int k = 2 * q + h;
+            const unsigned kk = __float_as_uint(h ? t.y : t.x) - 0x4B000000u;
+            in[k] = kk < n_last;
+            const float2* tr = trace + (in[k] ? static_cast<unsigned>(k * a.n_smp) + kk : 0u);
+            s0[k] = __ldg(tr);
+            s1[k] = __ldg(tr + 1);
+          }
+        }
 #pragma unroll
         for (int k = 0; k < kG; ++k) {
-          if (!(mask & (1u << k))) continue;
-          const float idx = (tau + rt[k] - a.t0) * a.fs;
-          const float fl = floorf(idx);
-          const int kk = static_cast<int>(fl);
-          if (static_cast<unsigned>(kk) >= n_last) continue;
-          const float f = idx - fl;
-          const float2* tr = trace + static_cast<long>(k) * a.n_smp + kk;
-          const float2 s0 = __ldg(tr), s1 = __ldg(tr + 1);
-          const float vr = fmaf(f, s1.x - s0.x, s0.x);
-          const float vi = fmaf(f, s1.y - s0.y, s0.y);
-          ar[k] = fmaf(wr, vr, fmaf(-wi, vi, ar[k]));
-          ai[k] = fmaf(wr, vi, fmaf(wi, vr, ai[k]));
+          const float f = (k & 1) ? f2[k / 2].y : f2[k / 2].x;
+          const float2 v = __ffma2_rn(make_float2(f, f), __ffma2_rn(s0[k], kMinus2, s1[k]), s0[k]);
+          const float2 t = make_float2(fmaf(-w2.y, v.y, acc[k].x), fmaf(w2.y, v.x, acc[k].y));
+          const float2 r = __ffma2_rn(wr2, v, t);
+          if (in[k]) acc[k] = r;
         }
       }
     }
     if (kSum) {
-      __syncthreads();   // the table is read for the last time
 #pragma unroll
       for (int k = 0; k < kG; ++k) {
         const int ch = g + k;
@@ -627,26 +693,25 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
         if ((mask >> k) & 1u) {
           const float ap = aperture_weight(elem_x(a, ch), px, pz, a.f_number, a.rx_window, a.tukey_alpha);
           float rc = 1.0f, rs = 0.0f;
-          if (a.fdem > 0.0f) sincosf(a.two_pi_f * rt[k], &rs, &rc);
+          if (a.fdem > 0.0f) sincosf(a.two_pi_f * ((k & 1) ? rt[k / 2].y : rt[k / 2].x), &rs, &rc);
           const float gr = ap * rc, gi = ap * rs;
-          y = make_float2(fmaf(gr, ar[k], -gi * ai[k]), fmaf(gr, ai[k], gi * ar[k]));
+          y = make_float2(fmaf(gr, acc[k].x, -gi * acc[k].y), fmaf(gr, acc[k].y, gi * acc[k].x));
         }
-        ys[(cq * kG + k) * (32 * kPW) + pl] = y;
+        ys[(cq * kG + k) * kPx + pl] = y;
       }
-      act_s[cq][pl] = mask;
+      act_s[cq * kPx + pl] = mask;
       __syncthreads();
-      // (The next pass's __syncthreads_or keeps the table's writers out of
-      // these values until the combine is done.)
+      // The channel combine of das_fast_tile, by channel warp 0's thread of
+      // each pixel over the pass's channels in ascending order.
       if (cq == 0 && valid) {
-        cplx das = mk(cs[0][pl], cs[1][pl]), s = mk(cs[2][pl], cs[3][pl]), q = mk(cs[4][pl], cs[5][pl]),
-             coh = mk(cs[6][pl], cs[7][pl]);
-        float incs = cs[8][pl];
-        int n_active = __float_as_int(cs[9][pl]);
+        cplx das = mk(cs[0 * kPx + pl], cs[1 * kPx + pl]), s = mk(cs[2 * kPx + pl], cs[3 * kPx + pl]),
+             q = mk(cs[4 * kPx + pl], cs[5 * kPx + pl]), coh = mk(cs[6 * kPx + pl], cs[7 * kPx + pl]);
+        float incs = cs[8 * kPx + pl];
+        int n_active = __float_as_int(cs[9 * kPx + pl]);
         for (int c = 0; c < kCQ * kG; ++c) {
-          const int ch = pass * kCQ * kG + c;
-          if (ch >= a.n_ch) break;
-          const bool act = (act_s[c / kG][pl] >> (c % kG)) & 1u;
-          const float2 yv = ys[c * (32 * kPW) + pl];
+          if (g0 * kG + c >= a.n_ch) break;
+          const bool act = (act_s[(c / kG) * kPx + pl] >> (c % kG)) & 1u;
+          const float2 yv = ys[c * kPx + pl];
           const cplx y = mk(yv.x, yv.y);
           n_active += act ? 1 : 0;
           if (a.combiner == USX_COMB_DMAS) {
@@ -664,20 +729,21 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
             incs += cnorm(y);
           }
         }
-        cs[0][pl] = das.re;
-        cs[1][pl] = das.im;
-        cs[2][pl] = s.re;
-        cs[3][pl] = s.im;
-        cs[4][pl] = q.re;
-        cs[5][pl] = q.im;
-        cs[6][pl] = coh.re;
-        cs[7][pl] = coh.im;
-        cs[8][pl] = incs;
-        cs[9][pl] = __int_as_float(n_active);
+        cs[0 * kPx + pl] = das.re;
+        cs[1 * kPx + pl] = das.im;
+        cs[2 * kPx + pl] = s.re;
+        cs[3 * kPx + pl] = s.im;
+        cs[4 * kPx + pl] = q.re;
+        cs[5 * kPx + pl] = q.im;
+        cs[6 * kPx + pl] = coh.re;
+        cs[7 * kPx + pl] = coh.im;
+        cs[8 * kPx + pl] = incs;
+        cs[9 * kPx + pl] = __int_as_float(n_active);
       }
+      __syncthreads();   // the pass's values are read: the next may write its own
       continue;
     }
-    if (!valid) continue;
+    if (!valid || grp >= g_hi) continue;
 #pragma unroll
     for (int k = 0; k < kG; ++k) {
       const int ch = g + k;
@@ -686,18 +752,18 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
       float2 y = make_float2(0.f, 0.f);
       if (act) {
         float rc = 1.0f, rs = 0.0f;
-        if (a.fdem > 0.0f) sincosf(a.two_pi_f * rt[k], &rs, &rc);
+        if (a.fdem > 0.0f) sincosf(a.two_pi_f * ((k & 1) ? rt[k / 2].y : rt[k / 2].x), &rs, &rc);
         const float gr = 1.0f * rc, gi = 1.0f * rs;   // the export carries no aperture weight
-        y = make_float2(fmaf(gr, ar[k], -gi * ai[k]), fmaf(gr, ai[k], gi * ar[k]));
+        y = make_float2(fmaf(gr, acc[k].x, -gi * acc[k].y), fmaf(gr, acc[k].y, gi * acc[k].x));
       }
       a.y_out[(frame * a.n_pix + pix) * a.n_ch + ch] = y;
     }
   }
   if (kSum && cq == 0 && valid) {
-    const cplx das = mk(cs[0][pl], cs[1][pl]), s = mk(cs[2][pl], cs[3][pl]), q = mk(cs[4][pl], cs[5][pl]),
-               coh = mk(cs[6][pl], cs[7][pl]);
-    const float incs = cs[8][pl];
-    const int n_active = __float_as_int(cs[9][pl]);
+    const cplx das = mk(cs[0 * kPx + pl], cs[1 * kPx + pl]), s = mk(cs[2 * kPx + pl], cs[3 * kPx + pl]),
+               q = mk(cs[4 * kPx + pl], cs[5 * kPx + pl]), coh = mk(cs[6 * kPx + pl], cs[7 * kPx + pl]);
+    const float incs = cs[8 * kPx + pl];
+    const int n_active = __float_as_int(cs[9 * kPx + pl]);
     cplx out;
     if (n_active == 0) {
       out = mk(0.f, 0.f);
@@ -713,15 +779,14 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
   }
 }
 
-template <int kG, int kPW, int kCQ, int kWL>
-__global__ void __launch_bounds__(32 * kPW * kCQ) das_export_kernel(const BfArgs a) {
-  das_export_body<kG, kPW, kCQ, kWL, false>(a, blockIdx.x, blockIdx.y);
+template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB>
+__global__ void __launch_bounds__(32 * kPW * kCQ, MB) das_export_kernel(const BfArgs a) {
+  das_export_body<kG, kPW, kCQ, kWL, kTL, false>(a, blockIdx.x, blockIdx.y);
 }
-// The channel-combining instance (delay-and-sum, DMAS, coherence factor):
-// three CTAs per SM, as the export's fastest shape runs.
-template <int kG, int kPW, int kCQ, int kWL>
-__global__ void __launch_bounds__(32 * kPW * kCQ, 3) das_csum_kernel(const BfArgs a) {
-  das_export_body<kG, kPW, kCQ, kWL, true>(a, blockIdx.x, blockIdx.y);
+// The channel-combining instance (delay-and-sum, DMAS, coherence factor).
+template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB>
+__global__ void __launch_bounds__(32 * kPW * kCQ, MB) das_csum_kernel(const BfArgs a) {
+  das_export_body<kG, kPW, kCQ, kWL, kTL, true>(a, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------------------
@@ -761,9 +826,9 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_queue_kernel(const 
   }
 }
 
-// The same queue over das_csum_kernel's body (IQ plans): CTAs of 4 pixel
-// warps x 4 channel warps on the same 4-line x 32-depth tiles.
-__global__ void __launch_bounds__(512, 3) das_csum_queue_kernel(const DasQueueArgs q) {
+// The same queue over das_csum_kernel's body (IQ plans): CTAs of 2 pixel
+// warps x 8 channel warps on 8-line x 8-depth tiles.
+__global__ void __launch_bounds__(512, 2) das_csum_queue_kernel(const DasQueueArgs q) {
   __shared__ int s_item;
   const int total = q.first[q.n];
   for (;;) {
@@ -776,7 +841,7 @@ __global__ void __launch_bounds__(512, 3) das_csum_queue_kernel(const DasQueueAr
     while (e + 1 < q.n && item >= q.first[e + 1]) ++e;
     const int local = item - q.first[e];
     const int frame = local / q.tiles[e], tile = local - frame * q.tiles[e];
-    das_export_body<4, 4, 4, 4, true>(q.args[e], tile, frame);
+    das_export_body<4, 2, 8, 4, 8, true>(q.args[e], tile, frame);
   }
 }
 
@@ -1665,6 +1730,7 @@ struct DasVariant {
   int producer_warps = 0;   // das_ring_kernel: one warp beside the tile's warps
   int channel_warps = 1;    // das_export_kernel: warps per pixel warp (IQ: MV exports, coherent sums; else variant 0)
   void (*sum)(BfArgs) = nullptr;   // das_csum_kernel, the channel-combining instance (plain IQ launches)
+  int grid_lines = 0;       // das_export_kernel: lines of the tile (32 x pixel warps / grid_lines depths)
 };
 // RF input (the reference's interp_rf path) keeps the default shape in
 // every variant.
@@ -1683,13 +1749,12 @@ template <int G, int TL, int E>
 constexpr DasVariant das_staged_variant() {
   return DasVariant{G, TL, 0, 1, false, das_staged_kernel<G, TL, E>, das_fast_kernel<false, 16, 4, 1>, true, false};
 }
-// The channel-warp kernel: minimum-variance exports, and coherent or select
-// IQ delay-and-sum, DMAS and coherence factor with the channel combine in
-// shared memory; RF and incoherent launches use variant 0.
-template <int G, int PW, int CQ, int WL>
+// The channel-warp kernels (traces of 2 to 2^23 samples); RF and incoherent
+// launches use variant 0.
+template <int G, int PW, int CQ, int WL, int TL, int MB>
 constexpr DasVariant das_export_variant() {
-  return DasVariant{G, PW, 0, WL, false, das_export_kernel<G, PW, CQ, WL>, das_fast_kernel<false, 16, 4, 1>,
-                    false, false, 0, CQ, das_csum_kernel<G, PW, CQ, WL>};
+  return DasVariant{G, PW, 0, WL, false, das_export_kernel<G, PW, CQ, WL, TL, MB>, das_fast_kernel<false, 16, 4, 1>,
+                    false, false, 0, CQ, das_csum_kernel<G, PW, CQ, WL, TL, MB>, TL};
 }
 // The producer-warp ring (same applicability as the staged kernel).
 template <int G, int TL, int S>
@@ -1697,7 +1762,7 @@ constexpr DasVariant das_ring_variant() {
   return DasVariant{G, TL, 0, 1, false, das_ring_kernel<G, TL, S>, das_fast_kernel<false, 16, 4, 1>, true, false, 1};
 }
 const DasVariant kDasVariants[] = {
-    das_variant<8, 4, 8>(),  das_variant<16, 4, 1>(), das_variant<16, 8, 2>(), das_variant<32, 4, 1>(),
+    das_variant<8, 4, 8>(),  das_export_variant<4, 1, 8, 4, 4, 4>(), das_export_variant<4, 2, 4, 4, 8, 4>(), das_export_variant<4, 1, 32, 4, 4, 1>(),
     das_variant<8, 8, 4>(),  das_variant<16, 2, 8>(), das_variant<4, 4, 12>(), das_variant<8, 2, 16>(),
     das_variant<16, 4, 8, true>(), das_variant<16, 2, 16, true>(), das_staged_variant<8, 4, 1>(),
     das_variant<8, 4, 8, false, 4>(), das_variant<4, 4, 12, false, 4>(), das_variant<4, 4, 12, false, 2>(),
@@ -1706,9 +1771,39 @@ const DasVariant kDasVariants[] = {
     das_variant<8, 4, 8, false, 4, true>(),
     das_table_variant<4, 2, 2>(),
     das_ring_variant<8, 8, 8>(),
-    das_export_variant<4, 4, 4, 4>(), das_export_variant<8, 4, 4, 4>(),
+    das_export_variant<4, 4, 4, 4, 4, 2>(), das_export_variant<4, 2, 8, 4, 8, 2>(),
 };
 constexpr int kNumDasVariants = static_cast<int>(sizeof(kDasVariants) / sizeof(kDasVariants[0]));
+
+// Dynamic shared memory of a channel-warp launch whose frames have `events`
+// events each, and the events its table holds.
+size_t channel_warp_smem(const DasVariant& v, int events, bool sum, int* tab_events) {
+  *tab_events = std::max(1, std::min(events, kTabEvents));
+  return exp_smem_bytes(*tab_events, v.tile_lines, v.channel_warps, v.group, sum);
+}
+// The channel-warp kernels take traces of 2 to 2^23 samples (floor by a
+// directed-rounding addition; a pair load needs two samples).
+bool channel_warp_samples(int n_smp) { return n_smp >= 2 && n_smp <= kMaxFastSamples; }
+
+// The shape of a plan whose variant was neither set nor tuned (IQ, coherent or
+// select). Measured at 128 channels (us; shapes by index):
+//   at most one 32-pixel tile per SM: all channels at once (3), the rest wait
+//     on one tile's latency;
+//   up to 48 Ki pixels: 32-pixel tiles (1) fill the SMs: 11 events, 128 x 256
+//     pixels, 61 against 74 (2) and 86 (22); 128 x 512, 105 / 99 / 95;
+//   more than 56 events: the table of a larger tile leaves too few CTAs per SM
+//     (256 x 512 pixels, 56 events: 570 (1), 548 (2), 559 (22); 64 events:
+//     638, 718, 1024);
+//   up to 16 events: 128-pixel tiles (22) share the traces best (3 events:
+//     145 (1), 123 (2), 111 (22); 24 events: 296, 269, 271);
+//   else 64-pixel tiles (2).
+int default_variant(int n0, int n1, int n_frames, int events, int sm_count) {
+  const long tiles = static_cast<long>(ceil_div(n0, 4)) * ceil_div(n1, 8) * n_frames;
+  const long pixels = static_cast<long>(n0) * n1 * n_frames;
+  if (tiles <= sm_count) return 3;
+  if (pixels <= 48 * 1024 || events > 56) return 1;
+  return events <= 16 ? 22 : 2;
+}
 
 // ------------------------------------------------------------------------
 // Minimum variance (reference beamformer.cpp:137-214, Cholesky :47-79).
@@ -1921,7 +2016,8 @@ struct usx_bf_plan {
   int ev_begin = 0, ev_end = 0;
   int mv_mode = USX_MV_EXACT;
   int precision = USX_BF_FAST;
-  int das_variant = 0;         // index into kDasVariants (the autotuner's choice)
+  int das_variant = 0;         // index into kDasVariants (set by the caller or the autotuner)
+  bool variant_set = false;    // false: default_variant's rule picks the shape
   bool all_plane_waves = false;  // every event is a plane wave (the staged kernel's bound)
   int* d_mv_stats = nullptr;   // [0] FP64 re-solves, [1] factorisation failures, [2] learned-MV gate rejections
   // Learned minimum variance: the network (not owned) and the gate on |1^H w - 1|.
@@ -2064,7 +2160,11 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
     return USX_OK;
   }
   const bool fast = plan->precision == USX_BF_FAST;
-  const DasVariant* dvp = &kDasVariants[plan->das_variant];
+  const bool plain_iq = plan->cd.is_iq && a.compounding != USX_COMP_INCOHERENT;
+  const DasVariant* dvp = &kDasVariants[!plan->variant_set && plain_iq
+                                            ? default_variant(plan->n0, plan->n1, n_frames, ev_per_frame, ctx->sm_count)
+                                            : plan->das_variant];
+  if (dvp->channel_warps > 1 && !channel_warp_samples(a.n_smp)) dvp = &kDasVariants[0];
   if (dvp->staged) {
     const bool ok = plan->cd.is_iq && plan->all_plane_waves && a.compounding != USX_COMP_INCOHERENT &&
                     reinterpret_cast<uintptr_t>(data) % 16 == 0 && a.n_smp >= kStageW + 2;
@@ -2077,6 +2177,8 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
   const DasVariant& dv = *dvp;
   const bool table = fast && dv.table;
   dim3 grid_das(table  ? ceil_div(plan->n0, dv.warp_lines) * ceil_div(plan->n1, 32 / dv.warp_lines)
+                : fast && dv.grid_lines
+                    ? ceil_div(plan->n0, dv.grid_lines) * ceil_div(plan->n1, 32 * dv.tile_lines / dv.grid_lines)
                 : fast ? ceil_div(plan->n0, dv.tile_lines) * ceil_div(plan->n1, 32)
                        : ceil_div(n_pix, kBfThreads),
                 n_frames);
@@ -2087,12 +2189,14 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
     const bool csum = fast && dv.channel_warps > 1 && !b.is_mv && plan->cd.is_iq &&
                       !(b.compounding == USX_COMP_INCOHERENT && b.pass < 0);
     const bool cexport = fast && dv.channel_warps > 1 && b.is_mv && plan->cd.is_iq;
+    const int ev_per_launch = b.pass >= 0 ? 1 : ev_per_frame;
     // The profiling label names the kernel that runs.
     prof_begin(ctx, csum ? "das_csum_kernel" : cexport ? "das_export_kernel(mv export)" : name);
     if (csum) {
-      const size_t tb = exp_table_bytes(dv.tile_lines);
+      BfArgs t = b;
+      const size_t tb = channel_warp_smem(dv, ev_per_launch, true, &t.tab_events);
       if (int rc_ = smem_limit(reinterpret_cast<const void*>(dv.sum), tb)) return rc_;
-      dv.sum<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(b);
+      dv.sum<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
     } else if (fast && dv.channel_warps > 1 && !(b.is_mv && plan->cd.is_iq)) {
       // A channel-warp shape on an RF or incoherent launch: variant 0.
       const DasVariant& d0 = kDasVariants[0];
@@ -2102,9 +2206,10 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
       else
         d0.rf<<<g0, 32 * d0.tile_lines, 0, ctx->stream>>>(b);
     } else if (fast && dv.channel_warps > 1) {
-      const size_t tb = exp_table_bytes(dv.tile_lines);
+      BfArgs t = b;
+      const size_t tb = channel_warp_smem(dv, ev_per_launch, false, &t.tab_events);
       if (int rc_ = smem_limit(reinterpret_cast<const void*>(dv.iq), tb)) return rc_;
-      dv.iq<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(b);
+      dv.iq<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
     } else if (table) {
       dv.iq<<<grid_das, 32 * table_warps(dv.group, b.n_ch), table_smem, ctx->stream>>>(b);
     } else if (fast) {
@@ -2471,6 +2576,7 @@ int usx_cu_bf_plan_set_variant(usx_bf_plan* plan, int index) {
   if (!plan) return fail(USX_ERR_INVALID, "usx_cu_bf_plan_set_variant: null plan");
   if (index < 0 || index >= kNumDasVariants) return fail(USX_ERR_INVALID, "usx_cu_bf_plan_set_variant: no such variant");
   plan->das_variant = index;
+  plan->variant_set = true;
   return USX_OK;
 }
 
@@ -2489,6 +2595,7 @@ int usx_cu_bf_plan_autotune(usx_bf_plan* plan, const void* data, float* frame, i
   USX_CUDA(cudaEventCreate(&e0));
   USX_CUDA(cudaEventCreate(&e1));
   int best = plan->das_variant;
+  plan->variant_set = true;
   float best_ms = 0.0f;
   int rc = USX_OK;
   const bool saved_prof = ctx->profiling;
@@ -2645,6 +2752,10 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     std::memset(&q, 0, sizeof(q));
     q.n = 0;
     q.first[0] = 0;
+    int tab_events = 1;
+    // Traces the channel-warp body does not take go to das_fast_kernel's tiles.
+    bool cw = iq;
+    for (int k = 0; k < m; ++k) cw = cw && channel_warp_samples(plans[i0 + k]->cd.acq.n_samples);
     for (int k = 0; k < m; ++k) {
       const usx_bf_plan* p = plans[i0 + k];
       BfArgs a = make_args(p);
@@ -2659,8 +2770,9 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
         USX_CUDA(cudaMemsetAsync(frames[i0 + k], 0, sizeof(float2) * a.n_pix, ctx->stream));
         continue;
       }
-      const int tiles = ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
+      const int tiles = cw ? ceil_div(p->n0, 8) * ceil_div(p->n1, 8) : ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
       q.args[q.n] = a;
+      tab_events = std::max(tab_events, std::min(kTabEvents, a.ev_end - a.ev_begin));
       q.tiles[q.n] = tiles;
       q.first[q.n + 1] = q.first[q.n] + tiles;
       ++q.n;
@@ -2668,21 +2780,24 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     if (q.n == 0) continue;
     q.next = next;
     USX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream));
-    // IQ: das_csum_kernel's body (4 pixel warps x 4 channel warps, the
-    // transmit table, the in-order channel combine; the autotuner's usual
-    // choice); RF: das_fast_kernel's RF shape.
-    const void* kern = iq ? reinterpret_cast<const void*>(das_csum_queue_kernel)
-                          : reinterpret_cast<const void*>(das_queue_kernel<false, 16, 4, 1>);
-    const int threads = iq ? 512 : 32 * 4;
-    const size_t tb = iq ? exp_table_bytes(4) : 0;
-    if (iq)
+    // IQ: das_csum_kernel's body (2 pixel warps x 8 channel warps); RF, and
+    // traces that body does not take: das_fast_kernel's shape.
+    const void* kern = cw   ? reinterpret_cast<const void*>(das_csum_queue_kernel)
+                       : iq ? reinterpret_cast<const void*>(das_queue_kernel<true, 16, 4, 1>)
+                            : reinterpret_cast<const void*>(das_queue_kernel<false, 16, 4, 1>);
+    const int threads = cw ? 512 : 32 * 4;
+    const size_t tb = cw ? exp_smem_bytes(tab_events, 2, 8, 4, true) : 0;
+    for (int k = 0; k < q.n; ++k) q.args[k].tab_events = tab_events;
+    if (cw)
       if (int rc = smem_limit(kern, tb)) return rc;
     int per_sm = 0;
     if (int rc = occupancy(kern, threads, tb, &per_sm)) return rc;
     const unsigned grid = static_cast<unsigned>(std::max(1, per_sm) * ctx->sm_count);
-    prof_begin(ctx, iq ? "das_csum_queue_kernel" : "das_queue_kernel");
-    if (iq)
+    prof_begin(ctx, cw ? "das_csum_queue_kernel" : "das_queue_kernel");
+    if (cw)
       das_csum_queue_kernel<<<grid, threads, tb, ctx->stream>>>(q);
+    else if (iq)
+      das_queue_kernel<true, 16, 4, 1><<<grid, threads, 0, ctx->stream>>>(q);
     else
       das_queue_kernel<false, 16, 4, 1><<<grid, threads, 0, ctx->stream>>>(q);
     prof_end(ctx);
