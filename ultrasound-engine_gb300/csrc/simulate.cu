@@ -24,17 +24,28 @@
 // fixed-point step is 2^-61 of the bound on any sum (for realistic phantoms
 // well below the float rounding of a sample).
 //
+// What bounds it: instruction issue at 24 warps per SM (65% of the slots; about
+// 28,000 warp instructions per scatterer and event at 128 elements, 20,000 of
+// them in the echoes). Neither the reductions nor the shared-memory conflicts
+// of the echo reads do: leaving out either measured within 2%. 100,000
+// scatterers, 75 events x 128 elements: 316 ms with one sample per lane and
+// step behind four branches; 236 ms with the samples of an element in
+// independent FP32 pairs, the cell by a directed-rounding addition, predicated
+// reductions, one 16-byte table entry per element, and the incident field's
+// taps in registers on a path without bounds tests for elements whose pulse
+// lies inside the window.
+//
 // Occupancy: a warp keeps a 1,536-sample incident buffer and element tables
 // sized to the probe in shared memory (8 KB at 128 elements), so that eight
 // warps per CTA and three CTAs per SM fit; windows longer than the buffer
-// (up to the 30 us clamp) use the warp's slot of a global buffer through the
-// same generic pointer, and the grid is persistent over (event, block of
-// scatterers) items so that there is one slot per resident warp. Against
-// buffers sized for the clamp (10 warps per SM): 509 -> 311 ms for 100,000
-// scatterers. The fixed-point scale (a power of two) is folded into each
-// element's amplitude, which gives the same scaled samples exactly. A
-// 960-sample buffer with a register cap for four CTAs per SM (58 registers)
-// measured slower (356 ms).
+// (6% of the pairs, up to the 30 us clamp) use the warp's slot of a global
+// buffer, and the grid is persistent over (event, block of scatterers) items
+// so that there is one slot per resident warp. The fixed-point scale (a power
+// of two) is folded into each element's amplitude, which gives the same scaled
+// samples exactly. Measured slower: four CTAs per SM with 1,280-sample buffers
+// and the sample times in global memory (292 ms); the long windows in a second
+// pass with buffers for the clamp (249 to 269 ms at 768 to 1,536 samples for
+// the first); the 64-bit conversion by additions (253 ms; half of them, 238).
 //
 // Measured and dropped (100,000 scatterers, 75 events x 128 elements, 509 ms
 // for the kernel at the time): the incident waveforms of a batch written to a pool and
@@ -62,6 +73,7 @@ constexpr int kMaxTimeTable = 8192;
 // Incident samples a warp keeps in shared memory; a longer window (up to the
 // clamp) uses the warp's slot of a global-memory buffer instead.
 constexpr int kIncSmall = 1536;
+constexpr int kTimeSlack = 128;   // sample times past the record (read, not used)
 
 struct SimArgs {
   const usx_scatterer* scat;
@@ -124,27 +136,83 @@ __device__ __forceinline__ int fixed_shift(const SimArgs& a) {
   return 61 - e;
 }
 
+// at[0] += v where n <= n1, k <= last and u > -1: a predicated reduction, no
+// branch around it.
+__device__ __forceinline__ void red_add(unsigned long long* at, unsigned long long v, int n, int n1, unsigned k,
+                                        unsigned last, float u) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.le.s32 p, %2, %3;\nsetp.le.and.u32 p, %4, %5, p;\n"
+      "setp.gt.and.f32 p, %6, 0fBF800000, p;\n@p red.global.add.u64 [%0], %1;\n}\n"
+      :: "l"(at), "l"(v), "r"(n), "r"(n1), "r"(k), "r"(last), "f"(u) : "memory");
+}
+
+// One receive element's echo of the trimmed waveform tr[trim_n].
+struct EchoArgs {
+  const float* tr;
+  const float* t_axis;     // sample times (kTable)
+  unsigned long long* dst; // the element's accumulator row
+  float amp, delay, trim_t0, fs_os, t0, fs;
+  int n1, trim_n;
+};
+
+// Samples n and (kPair) n + 32 of an element, most of the arithmetic on FP32
+// pairs: u = (t - delay - trim_t0) fs_os, the cell trunc(u) by a
+// directed-rounding addition (0 for u in (-1, 0)), the interpolated value
+// scaled by amp. (The interpolation's sum is scalar: a packed sum would be
+// fused with the packed product before it.)
+template <bool kPair, bool kTable>
+__device__ __forceinline__ void echo_samples(const EchoArgs& q, int na) {
+  const float2 neg_delay = make_float2(-q.delay, -q.delay), neg_t0 = make_float2(-q.trim_t0, -q.trim_t0);
+  const float2 os2 = make_float2(q.fs_os, q.fs_os), amp2 = make_float2(q.amp, q.amp);
+  const float2 big = make_float2(8388608.0f, 8388608.0f), minus = make_float2(-1.0f, -1.0f);
+  const unsigned last = static_cast<unsigned>(q.trim_n - 2);   // (trim_n >= 2)
+  const int nb = kPair ? na + 32 : na;
+  const float2 t = kTable ? make_float2(q.t_axis[na], q.t_axis[nb])
+                          : make_float2(q.t0 + static_cast<float>(na) / q.fs, q.t0 + static_cast<float>(nb) / q.fs);
+  const float2 u = __fmul2_rn(__fadd2_rn(__fadd2_rn(t, neg_delay), neg_t0), os2);
+  float2 w = __fadd2_rd(u, big);
+  w.x = fmaxf(w.x, 8388608.0f);
+  w.y = fmaxf(w.y, 8388608.0f);
+  const float2 f = __fadd2_rn(u, __ffma2_rn(w, minus, big));   // u - trunc(u)
+  const unsigned ka = __float_as_uint(w.x) - 0x4B000000u, kb = __float_as_uint(w.y) - 0x4B000000u;
+  const float* ta = q.tr + min(ka, last);
+  const float* tb = q.tr + min(kb, last);
+  const float2 va = make_float2(ta[0], tb[0]), vb = make_float2(ta[1], tb[1]);
+  const float2 d = __fmul2_rn(__ffma2_rn(va, minus, vb), f);
+  const float2 v = __fmul2_rn(amp2, make_float2(va.x + d.x, va.y + d.y));
+  red_add(q.dst + na, static_cast<unsigned long long>(__float2ll_rn(v.x)), na, q.n1, ka, last, u.x);
+  if (kPair) red_add(q.dst + nb, static_cast<unsigned long long>(__float2ll_rn(v.y)), nb, q.n1, kb, last, u.y);
+}
+
+template <bool kTable>
 __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs a) {
   extern __shared__ float4 sim_smem[];
-  // Shared memory: the pulse, the sample-time table, then per warp a small
-  // incident buffer and four element tables (sized to the probe).
-  float* pulse = reinterpret_cast<float*>(sim_smem);
-  float* t_axis = pulse + a.pulse_pad;
+  // Shared memory: per warp an element table and a small incident buffer, then
+  // the pulse and the sample-time table (read up to 127 past its end by lanes
+  // that store nothing; kTimeSlack words follow it).
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per_warp = a.inc_small + 4 * a.tbl_pad;
-  float* mine = t_axis + (a.t_table ? a.n_smp + (4 - a.n_smp % 4) % 4 : 0) + warp * per_warp;
-  float* inc_smem = mine;                       // [inc_small]
+  float4* e_tab = sim_smem + warp * (a.inc_small / 4 + a.tbl_pad);   // [tbl_pad]
+  float* inc_smem = reinterpret_cast<float*>(e_tab + a.tbl_pad);     // [inc_small]
+  float* pulse = reinterpret_cast<float*>(sim_smem + kSimWarps * (a.inc_small / 4 + a.tbl_pad));
+  float* t_axis = pulse + a.pulse_pad;
   float* inc_glob = a.inc_global + (static_cast<long>(blockIdx.x) * kSimWarps + warp) * a.inc_cap;
-  float* e_r = inc_smem + a.inc_small;          // distance to each element
-  float* e_amp = e_r + a.tbl_pad;               // stage-1 amplitude (active order)
-  float* e_ctr = e_amp + a.tbl_pad;             // stage-1 centre index (active order)
-  int* e_base = reinterpret_cast<int*>(e_ctr + a.tbl_pad);
   for (int k = threadIdx.x; k < a.pulse_n; k += blockDim.x) pulse[k] = a.pulse[k];
   // Sample times t0 + n / fs of the RF axis, each computed as the reference
   // does (float division), once per block instead of once per echo sample.
-  if (a.t_table)
-    for (int n = threadIdx.x; n < a.n_smp; n += blockDim.x) t_axis[n] = a.t0 + static_cast<float>(n) / a.fs;
+  if (kTable)
+    for (int n = threadIdx.x; n < a.n_smp + kTimeSlack; n += blockDim.x)
+      t_axis[n] = a.t0 + static_cast<float>(n) / a.fs;
   __syncthreads();
+  // A slot j of the pulse's stretch takes the "next sample" term of tap j - 1
+  // and the "this sample" term of tap j. Up to 64 slots the lane's taps stay
+  // in registers, zero past the pulse's ends (adding zero changes nothing).
+  const bool short_pulse = a.pulse_n < 64;
+  float2 taps[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int j = lane + 32 * h;
+    taps[h] = make_float2(j >= 1 && j <= a.pulse_n ? pulse[j - 1] : 0.0f, j < a.pulse_n ? pulse[j] : 0.0f);
+  }
 
   // 2^shift as two float factors, each within float range whatever the bound.
   const int shift = fixed_shift(a);
@@ -175,19 +243,14 @@ __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs 
       pz = pz + sc.vz * event_time;
     }
     if (pz <= 0.0f) continue;
-
-    // Distances to every element.
-    for (int e = lane; e < a.n_el; e += 32) {
-      const float ex = (static_cast<float>(e) - a.half_nm1) * a.pitch;
-      e_r[e] = dist3(px, py, pz, ex, 0.0f, 0.0f);
-    }
-    __syncwarp();
+    auto elem_x = [&](int e) { return (static_cast<float>(e) - a.half_nm1) * a.pitch; };
+    auto distance = [&](int e) { return dist3(px, py, pz, elem_x(e), 0.0f, 0.0f); };
 
     // ---- stage 1: arrival span over firing elements -----------------------
     float t_min = INFINITY, t_max = -INFINITY;
     for (int q = lane; q < n_act; q += 32) {
       const int e = act[q];
-      const float t = dly[e] + e_r[e] / a.c;
+      const float t = dly[e] + distance(e) / a.c;
       t_min = fminf(t_min, t);
       t_max = fmaxf(t_max, t);
     }
@@ -201,48 +264,52 @@ __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs 
     const int inc_n = static_cast<int>(ceilf(span * a.fs_os)) + 2;
     if (inc_n > a.inc_cap || inc_n <= 0) continue;  // cannot happen: cap bounds the window
     // The window in shared memory when it fits, else in the warp's global slot
-    // (the same code through a generic pointer).
-    float* inc = inc_n <= a.inc_small ? inc_smem : inc_glob;
+    // (the same code, compiled for each address space).
+    auto field_and_echo = [&](float* inc) {
     for (int k = lane; k < inc_n; k += 32) inc[k] = 0.0f;
 
     // Per firing element: amplitude and pulse placement.
     for (int q = lane; q < n_act; q += 32) {
       const int e = act[q];
-      const float r = e_r[e];
+      const float r = distance(e);
       float amp = 0.0f;
       float centre = 0.0f;
       if (!(r < 1e-6f)) {
-        const float ex = (static_cast<float>(e) - a.half_nm1) * a.pitch;
-        amp = elem_amp(a, apd[e], px, ex, r);
+        amp = elem_amp(a, apd[e], px, elem_x(e), r);
         const float t_arr = dly[e] + r / a.c;
         centre = (t_arr - inc_t0) * a.fs_os;
-      } else {
-        amp = 0.0f;
       }
-      e_amp[q] = (r < 1e-6f) ? 0.0f : amp;
-      e_ctr[q] = centre;
-      e_base[q] = static_cast<int>(floorf(centre)) - a.pulse_n / 2;
+      const float whole = floorf(centre), frac = centre - whole;
+      e_tab[q] = make_float4(amp, frac, 1.0f - frac, __int_as_float(static_cast<int>(whole) - a.pulse_n / 2));
     }
     __syncwarp();
     for (int q = 0; q < n_act; ++q) {
-      const float amp = e_amp[q];
+      const float4 el = e_tab[q];
+      const float amp = el.x, frac = el.y, omf = el.z;
+      const int base = __float_as_int(el.w);
       if (amp == 0.0f) continue;
-      const float centre = e_ctr[q];
-      const int base = e_base[q];
-      const float frac = centre - floorf(centre);
-      const float omf = 1.0f - frac;
       // One lane per buffer slot s = base + j: first the "next sample" term of
       // tap j - 1, then the "this sample" term of tap j, which is the order in
       // which the reference's serial tap loop updates slot s (see header).
-      for (int j = lane; j <= a.pulse_n; j += 32) {
-        const int s = base + j;
-        const bool nx = j >= 1 && s >= 1 && s < inc_n;          // tap j - 1 at index s - 1
-        const bool th = j < a.pulse_n && s >= 0 && s + 1 < inc_n; // tap j at index s
-        if (!nx && !th) continue;
-        float t = inc[s];
-        if (nx) t += (amp * pulse[j - 1]) * frac;
-        if (th) t += (amp * pulse[j]) * omf;
-        inc[s] = t;
+      if (short_pulse && base >= 0 && base + a.pulse_n + 1 < inc_n) {
+        const float2 amp2 = make_float2(amp, amp), part = make_float2(frac, omf);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int j = lane + 32 * h;
+          const float2 term = __fmul2_rn(__fmul2_rn(amp2, taps[h]), part);
+          if (j <= a.pulse_n) inc[base + j] = (inc[base + j] + term.x) + term.y;
+        }
+      } else {
+        for (int j = lane; j <= a.pulse_n; j += 32) {
+          const int s = base + j;
+          const bool nx = j >= 1 && s >= 1 && s < inc_n;          // tap j - 1 at index s - 1
+          const bool th = j < a.pulse_n && s >= 0 && s + 1 < inc_n; // tap j at index s
+          if (!nx && !th) continue;
+          float t = inc[s];
+          if (nx) t += (amp * pulse[j - 1]) * frac;
+          if (th) t += (amp * pulse[j]) * omf;
+          inc[s] = t;
+        }
       }
       __syncwarp();
       if (!a.full) break;
@@ -252,35 +319,40 @@ __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs 
     float peak = 0.0f;
     for (int k = lane; k < inc_n; k += 32) peak = fmaxf(peak, fabsf(inc[k]));
     for (int o = 16; o > 0; o >>= 1) peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, o));
-    if (peak <= 0.0f) continue;
+    if (peak <= 0.0f) return;
     const float thr = peak * a.trim_amp;
-    int lo = inc_n, hi = -1;
-    for (int k0 = 0; k0 < inc_n; k0 += 32) {
+    // First and last sample that is kept, from either end.
+    auto kept = [&](int k0) {
       const int k = k0 + lane;
-      const bool keep = k < inc_n && !(fabsf(inc[k]) < thr);
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (m) {
-        lo = min(lo, k0 + __ffs(m) - 1);
-        hi = max(hi, k0 + 31 - __clz(m));
+      return __ballot_sync(0xffffffffu, k < inc_n && !(fabsf(inc[k]) < thr));
+    };
+    int lo = inc_n, hi = -1;
+    for (int k0 = 0; k0 < inc_n; k0 += 32)
+      if (const unsigned m = kept(k0)) {
+        lo = k0 + __ffs(m) - 1;
+        break;
       }
-    }
-    if (lo >= inc_n || hi <= lo) continue;
+    for (int k0 = (inc_n - 1) / 32 * 32; k0 >= 0; k0 -= 32)
+      if (const unsigned m = kept(k0)) {
+        hi = k0 + 31 - __clz(m);
+        break;
+      }
+    if (lo >= inc_n || hi <= lo) return;
     const float trim_t0 = inc_t0 + static_cast<float>(lo) / a.fs_os;
     const int trim_n = hi - lo + 1;
     const float* tr = inc + lo;
 
     // ---- stage 2: echo on every receive element ---------------------------------
     // Per receive element, one lane each: amplitude, delay and the echo's
-    // sample window (the stage-1 tables are free again; e_r[e] is read by
-    // the lane that then overwrites it with the window's last sample).
+    // sample window (the stage-1 table is free again).
     const float span_t = static_cast<float>(trim_n - 1) / a.fs_os;
+    __syncwarp();
     for (int e = lane; e < a.n_el; e += 32) {
-      const float r = e_r[e];
+      const float r = distance(e);
       float amp = 0.0f, delay = 0.0f;
       int n0 = 1, n1 = 0;
       if (!(r < 1e-6f)) {
-        const float ex = (static_cast<float>(e) - a.half_nm1) * a.pitch;
-        amp = elem_amp(a, sc.amplitude, px, ex, r);
+        amp = elem_amp(a, sc.amplitude, px, elem_x(e), r);
         if (amp != 0.0f) {
           delay = r / a.c;
           const float t_start = trim_t0 + delay;
@@ -297,28 +369,36 @@ __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs 
       }
       // The fixed-point scale is a power of two, so scaling the amplitude
       // gives the scaled sample exactly: amp 2^s x lerp = (amp x lerp) 2^s.
-      e_amp[e] = (amp * scale1) * scale2;
-      e_ctr[e] = delay;
-      e_base[e] = n0;
-      e_r[e] = __int_as_float(n1);
+      e_tab[e] = make_float4((amp * scale1) * scale2, delay, __int_as_float(n0), __int_as_float(n1));
     }
     __syncwarp();
+    EchoArgs q;
+    q.tr = tr;
+    q.t_axis = t_axis;
+    q.trim_t0 = trim_t0;
+    q.fs_os = a.fs_os;
+    q.t0 = a.t0;
+    q.fs = a.fs;
+    q.trim_n = trim_n;
     for (int e = 0; e < a.n_el; ++e) {
-      const int n0 = e_base[e], n1 = __float_as_int(e_r[e]);
-      if (n0 > n1) continue;
-      const float amp = e_amp[e], delay = e_ctr[e];
-      unsigned long long* dst = acc_ev + static_cast<long>(e) * a.n_smp;
-      for (int n = n0 + lane; n <= n1; n += 32) {
-        const float t = (a.t_table ? t_axis[n] : (a.t0 + static_cast<float>(n) / a.fs)) - delay;
-        const float u = (t - trim_t0) * a.fs_os;
-        const int k = static_cast<int>(u);
-        if (k < 0 || k + 1 >= trim_n) continue;
-        const float f = u - static_cast<float>(k);
-        const float va = tr[k], vb = tr[k + 1];
-        const float v = amp * (va + (vb - va) * f);
-        atomicAdd(dst + n, static_cast<unsigned long long>(__float2ll_rn(v)));
+      const float4 el = e_tab[e];
+      q.amp = el.x;
+      q.delay = el.y;
+      q.n1 = __float_as_int(el.w);
+      q.dst = acc_ev + static_cast<long>(e) * a.n_smp;
+      int n = __float_as_int(el.z);
+      for (; n + 96 <= q.n1; n += 128) {
+        echo_samples<true, kTable>(q, n + lane);
+        echo_samples<true, kTable>(q, n + 64 + lane);
       }
+      for (; n + 32 <= q.n1; n += 64) echo_samples<true, kTable>(q, n + lane);
+      if (n <= q.n1) echo_samples<false, kTable>(q, n + lane);
     }
+    };
+    if (inc_n <= a.inc_small)
+      field_and_echo(inc_smem);
+    else
+      field_and_echo(inc_glob);
     __syncwarp();
   }
   }  // work items
@@ -503,12 +583,13 @@ extern "C" int usx_cu_simulate(usx_ctx* ctx, const usx_channel_desc* cd,
   a.pulse_pad = (pulse_n + 3) / 4 * 4;
   a.tbl_pad = (n_el + 3) / 4 * 4;
   a.inc_small = std::min(kIncSmall, (inc_cap + 3) / 4 * 4);
-  const size_t smem = sizeof(float) * (a.pulse_pad + (a.t_table ? (n_smp + 3) / 4 * 4 : 0) +
+  const size_t smem = sizeof(float) * (a.pulse_pad + (a.t_table ? (n_smp + kTimeSlack + 3) / 4 * 4 : 0) +
                                        static_cast<size_t>(kSimWarps) * (a.inc_small + 4 * a.tbl_pad));
   if (smem > 227 * 1024) return fail(USX_ERR_UNSUPPORTED, "usx_cu_simulate: incident window too long");
-  if (int rc_ = smem_limit(reinterpret_cast<const void*>(simulate_kernel), static_cast<size_t>(static_cast<int>(smem)))) return rc_;
+  void (*const kernel)(SimArgs) = a.t_table ? simulate_kernel<true> : simulate_kernel<false>;
+  if (int rc_ = smem_limit(reinterpret_cast<const void*>(kernel), static_cast<size_t>(static_cast<int>(smem)))) return rc_;
   int per_sm = 0;
-  if (int rc_ = occupancy(reinterpret_cast<const void*>(simulate_kernel), 32 * kSimWarps, smem, &per_sm)) return rc_;
+  if (int rc_ = occupancy(reinterpret_cast<const void*>(kernel), 32 * kSimWarps, smem, &per_sm)) return rc_;
   const long grid = std::max<long>(1, std::min<long>(grid_max, static_cast<long>(std::max(1, per_sm)) * ctx->sm_count));
 
   if (n_scat > 0) {
@@ -517,7 +598,7 @@ extern "C" int usx_cu_simulate(usx_ctx* ctx, const usx_channel_desc* cd,
     USX_CUDA(cudaMemsetAsync(d_acc, 0, acc_bytes, ctx->stream));
     sim_bound_kernel<<<static_cast<unsigned>(ceil_div(n_scat, 256)), 256, 0, ctx->stream>>>(a);
     USX_CHECK_LAUNCH("sim_bound_kernel");
-    simulate_kernel<<<static_cast<unsigned>(grid), 32 * kSimWarps, smem, ctx->stream>>>(a);
+    kernel<<<static_cast<unsigned>(grid), 32 * kSimWarps, smem, ctx->stream>>>(a);
     prof_end(ctx);
     USX_CHECK_LAUNCH("simulate_kernel");
     fixed_to_float_kernel<<<static_cast<unsigned>(ceil_div(ev_size * n_ev, 256)), 256, 0, ctx->stream>>>(
