@@ -265,10 +265,23 @@ struct DispArgs {
   float* corr;
 };
 
-__global__ void displacement_kernel(const DispArgs p) {
-  const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (k >= static_cast<long>(p.n0) * p.n1) return;
-  const int i = static_cast<int>(k / p.n1), j = static_cast<int>(k - static_cast<long>(i) * p.n1);
+// The centre frequency of a pixel's phase slope along depth (the window's
+// axial autocorrelation), the demodulation frequency where it is implausible.
+__device__ __forceinline__ float disp_centre(const DispArgs& p, cplx R10) {
+  const float f_est = atan2f(R10.im, R10.re) * p.c / (4.0f * kPi * p.dz);
+  return (f_est > 0.25f * p.fdem && f_est < 2.0f * p.fdem) ? f_est : p.fdem;
+}
+
+// Correlation and displacement of a pixel from its best lag.
+__device__ __forceinline__ void disp_store(const DispArgs& p, long k, float corr, cplx R, int lag, float f_centre) {
+  p.corr[k] = fclamp(corr, 0.0f, 1.0f);
+  const float residual = -atan2f(R.im, R.re) * p.c / (4.0f * kPi * f_centre);
+  p.axial[k] = static_cast<float>(lag) * p.dz + residual;
+}
+
+// One pixel, any window and lag range, clipped to the grid.
+__device__ void disp_pixel(const DispArgs& p, int i, int j) {
+  const long k = static_cast<long>(i) * p.n1 + j;
   p.axial[k] = 0.0f;
   p.corr[k] = 0.0f;
   cplx R10 = mk(0.f, 0.f);
@@ -283,9 +296,7 @@ __global__ void displacement_kernel(const DispArgs p) {
       R10 = cadd(R10, cmul(cconj(mk(u.x, u.y)), mk(v.x, v.y)));
     }
   }
-  float f_centre = p.fdem;
-  const float f_est = atan2f(R10.im, R10.re) * p.c / (4.0f * kPi * p.dz);
-  if (f_est > 0.25f * p.fdem && f_est < 2.0f * p.fdem) f_centre = f_est;
+  const float f_centre = disp_centre(p, R10);
   if (f_centre <= 0.0f) return;
   cplx best_R = mk(0.f, 0.f);
   float best_corr = -1.0f;
@@ -317,9 +328,156 @@ __global__ void displacement_kernel(const DispArgs p) {
     }
   }
   if (best_corr < 0.0f) return;
-  p.corr[k] = fclamp(best_corr, 0.0f, 1.0f);
-  const float residual = -atan2f(best_R.im, best_R.re) * p.c / (4.0f * kPi * f_centre);
-  p.axial[k] = static_cast<float>(best_lag) * p.dz + residual;
+  disp_store(p, k, best_corr, best_R, best_lag, f_centre);
+}
+
+__global__ void displacement_kernel(const DispArgs p) {
+  const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  if (k >= static_cast<long>(p.n0) * p.n1) return;
+  const int i = static_cast<int>(k / p.n1);
+  disp_pixel(p, i, static_cast<int>(k - static_cast<long>(i) * p.n1));
+}
+
+// The same for kDispLines lateral lines per thread over the interior columns
+// [col_lo, col_hi), where no window of any lag is clipped in depth. There
+//   * the energy of `before` is one sum for all lags, and that of `after` at a
+//     lag is the unshifted window's at the shifted column, so both are formed
+//     once per pixel (the block's columns of `after` in shared memory);
+//   * a product a^* b at (line, depth) goes to every output of the thread whose
+//     window holds the line (up to 2 kKL + 1), and four lags share each load.
+// Every sum adds the same terms in the same (line, depth) order as disp_pixel,
+// so the maps are equal bit for bit. The first n_edge blocks take the other
+// columns, a pixel per thread, beside the interior blocks.
+// What bounds it: FP32 issue (the window sums' ordered additions). 256 x 1024,
+// 17 x 5 windows, 17 lags: 156 us; 501 us with a pixel per thread, which forms
+// its products and both energies anew for every lag.
+constexpr int kDispCols = 128, kDispLines = 4, kDispLags = 4;
+constexpr int kDispMaxLag = 1024;   // shared memory: 4 (128 + 2 lag_max) floats
+struct DispLines {
+  DispArgs p;
+  int col_lo, col_hi, col_blocks, n_edge;
+};
+template <int kKL>
+__global__ void __launch_bounds__(kDispCols) displacement_lines_kernel(const DispLines q) {
+  extern __shared__ float eb_s[];   // [kDispLines][kDispCols + 2 lag_max]
+  const DispArgs& p = q.p;
+  const int n1 = p.n1, ka = p.ka;
+  if (static_cast<int>(blockIdx.x) < q.n_edge) {
+    const int n_cols = n1 - (q.col_hi - q.col_lo);
+    const long m = static_cast<long>(blockIdx.x) * kDispCols + threadIdx.x;
+    if (m >= static_cast<long>(p.n0) * n_cols) return;
+    const int i = static_cast<int>(m / n_cols), c = static_cast<int>(m - static_cast<long>(i) * n_cols);
+    disp_pixel(p, i, c < q.col_lo ? c : c - q.col_lo + q.col_hi);
+    return;
+  }
+  const int blk = static_cast<int>(blockIdx.x) - q.n_edge;
+  const int i0 = blk / q.col_blocks * kDispLines, j0 = q.col_lo + blk % q.col_blocks * kDispCols;
+  const int j = j0 + threadIdx.x, width = kDispCols + 2 * p.lag_max;
+  // Term t(line, depth) into the sums of the lines whose windows hold it.
+  for (int c = threadIdx.x; c < width; c += kDispCols) {
+    const int col = j0 - p.lag_max + c;
+    float e[kDispLines] = {};
+    if (col + ka < n1) {   // (col - ka >= 0 for every interior column and lag)
+#pragma unroll
+      for (int l = 0; l < kDispLines + 2 * kKL; ++l) {
+        const int ii = i0 - kKL + l;
+        if (ii < 0 || ii >= p.n0) continue;
+        const float2* b = p.b + static_cast<long>(ii) * n1 + col - ka;
+        for (int d = 0; d <= 2 * ka; ++d) {
+          const float2 v = b[d];
+          const float m = v.x * v.x + v.y * v.y;
+#pragma unroll
+          for (int r = 0; r < kDispLines; ++r)
+            if (l >= r && l <= r + 2 * kKL) e[r] += m;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kDispLines; ++r) eb_s[r * width + c] = e[r];
+  }
+  __syncthreads();
+  if (j >= q.col_hi) return;
+
+  float ea[kDispLines] = {}, f_centre[kDispLines], best[kDispLines];
+  float2 R10[kDispLines] = {}, best_R[kDispLines] = {};
+  int best_lag[kDispLines] = {};
+#pragma unroll
+  for (int l = 0; l < kDispLines + 2 * kKL; ++l) {
+    const int ii = i0 - kKL + l;
+    if (ii < 0 || ii >= p.n0) continue;
+    const float2* a = p.a + static_cast<long>(ii) * n1 + j - ka;
+    float2 u = a[0];
+    for (int d = 0; d <= 2 * ka; ++d) {
+      const float2 v = a[d + 1];
+      const float m = u.x * u.x + u.y * u.y;
+      const float2 t = make_float2(u.x * v.x + u.y * v.y, u.x * v.y - u.y * v.x);
+#pragma unroll
+      for (int r = 0; r < kDispLines; ++r)
+        if (l >= r && l <= r + 2 * kKL) {
+          ea[r] += m;
+          R10[r] = __fadd2_rn(R10[r], t);
+        }
+      u = v;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kDispLines; ++r) {
+    f_centre[r] = disp_centre(p, mk(R10[r].x, R10[r].y));
+    best[r] = -1.0f;
+  }
+  for (int l0 = -p.lag_max; l0 <= p.lag_max; l0 += kDispLags) {
+    float2 R[kDispLines][kDispLags] = {};
+#pragma unroll
+    for (int l = 0; l < kDispLines + 2 * kKL; ++l) {
+      const int ii = i0 - kKL + l;
+      if (ii < 0 || ii >= p.n0) continue;
+      const float2* a = p.a + static_cast<long>(ii) * n1 + j - ka;
+      const float2* b = p.b + static_cast<long>(ii) * n1;
+      const int c0 = j - ka + l0;   // column of the first depth at the first lag
+      float2 w[kDispLags];
+#pragma unroll
+      for (int x = 0; x < kDispLags; ++x) w[x] = b[min(c0 + x, n1 - 1)];
+#pragma unroll 4
+      for (int d = 0; d <= 2 * ka; ++d) {
+        const float2 u = a[d];
+#pragma unroll
+        for (int x = 0; x < kDispLags; ++x) {
+          const float2 t = make_float2(u.x * w[x].x + u.y * w[x].y, u.x * w[x].y - u.y * w[x].x);
+#pragma unroll
+          for (int r = 0; r < kDispLines; ++r)
+            if (l >= r && l <= r + 2 * kKL) R[r][x] = __fadd2_rn(R[r][x], t);
+        }
+#pragma unroll
+        for (int x = 0; x + 1 < kDispLags; ++x) w[x] = w[x + 1];
+        w[kDispLags - 1] = b[min(c0 + d + kDispLags, n1 - 1)];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kDispLags; ++x) {
+      const int lag = l0 + x;
+      if (lag > p.lag_max) break;
+#pragma unroll
+      for (int r = 0; r < kDispLines; ++r) {
+        const float eb = eb_s[r * width + static_cast<int>(threadIdx.x) + p.lag_max + lag];
+        if (ea[r] <= 0.0f || eb <= 0.0f) continue;
+        const float cr = cabsf_(mk(R[r][x].x, R[r][x].y)) / sqrtf(ea[r] * eb);
+        if (cr > best[r]) {
+          best[r] = cr;
+          best_R[r] = R[r][x];
+          best_lag[r] = lag;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kDispLines; ++r) {
+    if (i0 + r >= p.n0) continue;
+    const long k = static_cast<long>(i0 + r) * n1 + j;
+    p.axial[k] = 0.0f;
+    p.corr[k] = 0.0f;
+    if (!(f_centre[r] <= 0.0f) && !(best[r] < 0.0f))
+      disp_store(p, k, best[r], mk(best_R[r].x, best_R[r].y), best_lag[r], f_centre[r]);
+  }
 }
 
 __global__ void strain_kernel(const float* axial, int n0, int n1, float dz, int half, float* strain) {
@@ -345,6 +503,16 @@ __global__ void strain_kernel(const float* axial, int n0, int n1, float dz, int 
     if (!(fabsf(denom) < 1e-20f)) out = (static_cast<float>(n) * sxy - sx * sy) / denom;
   }
   strain[k] = out;
+}
+
+// Whether the four-line kernel pays (window terms x lags per pixel; us, a pixel
+// per thread against four lines): 64 x 256 pixels, 225 terms 33 / 41, 243
+// terms 35 / 33; 256 x 512, 9 terms 19 / 23, 63 terms 29 / 29, 243 terms 65 /
+// 41; 256 x 1024, 1,445 terms 513 / 169; 12 x 64, 1,445 terms 131 / 125: few
+// terms over few pixels only pay for the block's set-up.
+bool disp_lines_pay(const DispArgs& p, long n_pix) {
+  const double terms = (2.0 * p.ka + 1) * (2.0 * p.kl + 1) * (2.0 * p.lag_max + 1);
+  return p.kl <= 2 && (terms >= 1000.0 || terms * static_cast<double>(n_pix) >= 8.4e6);
 }
 
 float axial_step(const float* axis1, int n1) {
@@ -696,8 +864,24 @@ int usx_cu_axial_displacement(usx_ctx* ctx, const float* before, const float* af
   p.c = speed_of_sound;
   p.axial = axial;
   p.corr = correlation;
+  // Columns whose windows no lag clips in depth (nor the phase slope's next
+  // sample) go kDispLines lines to a thread.
+  DispLines q;
+  q.p = p;
+  const long reach = static_cast<long>(p.ka) + std::max(1, p.lag_max);
+  q.col_lo = static_cast<int>(std::min<long>(reach, n1));
+  q.col_hi = static_cast<int>(std::max<long>(q.col_lo, n1 - reach));
   prof_begin(ctx, "displacement_kernel");
-  displacement_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(p);
+  if (disp_lines_pay(p, n) && p.lag_max <= kDispMaxLag && q.col_hi > q.col_lo) {
+    q.col_blocks = ceil_div(q.col_hi - q.col_lo, kDispCols);
+    q.n_edge = ceil_div(static_cast<long>(n0) * (n1 - (q.col_hi - q.col_lo)), kDispCols);
+    const unsigned grid = static_cast<unsigned>(q.n_edge + static_cast<long>(q.col_blocks) * ceil_div(n0, kDispLines));
+    const size_t smem = sizeof(float) * kDispLines * (kDispCols + 2 * p.lag_max);
+    auto kern = p.kl == 0 ? displacement_lines_kernel<0> : p.kl == 1 ? displacement_lines_kernel<1> : displacement_lines_kernel<2>;
+    kern<<<grid, kDispCols, smem, ctx->stream>>>(q);
+  } else {
+    displacement_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(p);
+  }
   prof_end(ctx);
   USX_CHECK_LAUNCH("displacement_kernel");
   return USX_OK;
