@@ -98,3 +98,39 @@ def test_scan_extent_is_the_points_extent(gpu, n0, n1):
     got = ctx.scan_convert(img.data_ptr(), grid, 4, 4, 0.0, px.data_ptr())
     want = [np.nanmin(pts[:, 0]), np.nanmax(pts[:, 0]), np.nanmin(pts[:, 2]), np.nanmax(pts[:, 2])]
     assert np.array_equal(got, np.array(want, np.float32))
+
+
+@pytest.mark.parametrize("n,n0,n1,ka,kl,order", [
+    (8, 241, 515, 4, 1, 1),     # four lines per thread: ragged lines and depths
+    (33, 83, 500, 6, 2, 2),     # more than one row block of the wall filter
+    (9, 300, 140, 0, 2, 1),     # a window of one depth
+    (64, 65, 700, 3, 2, 0),     # the longest ensemble
+    (5, 20, 33, 4, 1, 1), (12, 40, 60, 2, 3, 1),   # a pixel per thread
+])
+def test_colour_flow_at_every_window(gpu, oracle, n, n0, n1, ka, kl, order):
+    """Maps against the oracle, whose sums run in the same order: power and
+    variance to 1e-5, gates equal but for pixels within rounding of one."""
+    torch, capi, ctx = gpu
+    rng = np.random.default_rng(n * n1)
+    ph = np.exp(1j * 0.5 * np.arange(n))[:, None, None] * np.exp(2j * np.arange(n1))[None, None]
+    ens = ph + 3.0 + 0.5 * (rng.normal(size=(n, n0, n1)) + 1j * rng.normal(size=(n, n0, n1)))
+    ens = ens.astype(np.complex64)
+    axis = (0.02 + 4.9e-5 * np.arange(n1)).astype(np.float32)
+    kw = dict(polynomial_order=order, kernel_axial=ka, kernel_lateral=kl)
+    d = torch.from_numpy(ens).cuda()
+    out = [torch.full((n0, n1), 7.0, device="cuda") for _ in range(3)] + \
+          [torch.full((n0, n1), 9, dtype=torch.uint8, device="cuda")]
+    ctx.color_flow(d.data_ptr(), n, n0, n1, axis, 5e6, 5e3, 1540.0, capi.doppler_config(**kw),
+                   *[o.data_ptr() for o in out])
+    vel, power, var, valid = (o.cpu().numpy() for o in out)
+    w = oracle.color_flow(ens, axis, 5e6, 5e3, 1540.0, O.doppler_config(**kw))
+    assert rel_l2(power, w[1]) < 1e-5 and rel_l2(var, w[2]) < 1e-5
+    assert (valid != w[3]).mean() <= 1e-3
+    both = (valid == 1) & (np.asarray(w[3]) == 1)
+    if both.any():   # (8 frames: the wall filter leaves no pixel coherent enough)
+        assert np.abs(vel - w[0])[both].max() <= 1e-4 * np.abs(w[0]).max()
+    batch = [torch.empty((2, n0, n1), dtype=o.dtype, device="cuda") for o in out]
+    ctx.color_flow_batch(d.data_ptr(), [n, n - 1], [0, 1], n0, n1, axis, 5e6, 5e3, 1540.0, capi.doppler_config(**kw),
+                         *[o.data_ptr() for o in batch])
+    for o, b in zip(out, batch):
+        assert torch.equal(o, b[0])

@@ -63,28 +63,71 @@ struct WallArgs {
   float M[kMaxEns * kMaxEns];
 };
 
-__global__ void wall_kernel(const WallArgs a) {
-  extern __shared__ float2 zs[];   // [n][blockDim]
-  const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (k >= a.n_pix) return;
-  for (int j = 0; j < a.n; ++j) zs[j * blockDim.x + threadIdx.x] = a.ens[j * a.n_pix + k];
-  float p = 0.0f;
-  for (int i = 0; i < a.n; ++i) {
-    cplx acc;
-    if (a.identity) {
-      const float2 z = zs[i * blockDim.x + threadIdx.x];
-      acc = mk(z.x, z.y);
-    } else {
-      acc = mk(0.f, 0.f);
-      for (int j = 0; j < a.n; ++j) {
-        const float2 z = zs[j * blockDim.x + threadIdx.x];
-        acc = cadd(acc, cscale(mk(z.x, z.y), a.M[i * a.n + j]));
+// The wall filter's shared memory: the block's ensembles z[n][kWallThreads],
+// then the projector transposed, Mt[j][i] with rows of kWallRows multiples.
+constexpr int kWallThreads = 128, kWallRows = 8;
+__host__ __device__ constexpr int wall_pitch(int n) { return (n + kWallRows - 1) / kWallRows * kWallRows; }
+__host__ __device__ constexpr size_t wall_smem(int n) {
+  return sizeof(float2) * n * kWallThreads + sizeof(float) * n * wall_pitch(n);
+}
+
+// One pixel's ensemble src[j * n_pix] through the n x n projector M: filtered
+// frame i goes to store(i, value), ascending i. Eight rows at a time share each
+// read of z and two 16-byte reads of Mt; every row sums over j in ascending
+// order, products and sums rounded separately. Every thread of the block calls
+// it (in: the pixel exists).
+template <typename Store>
+__device__ __forceinline__ void wall_pixel(float4* smem, const float2* src, long n_pix, int n, const float* M,
+                                           bool identity, bool in, Store store) {
+  float2* z = reinterpret_cast<float2*>(smem) + threadIdx.x;
+  float* Mt = reinterpret_cast<float*>(reinterpret_cast<float2*>(smem) + n * kWallThreads);
+  const int pitch = wall_pitch(n);
+  if (in)
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) z[j * kWallThreads] = __ldg(src + j * n_pix);
+  if (identity) {
+    if (in)
+      for (int i = 0; i < n; ++i) store(i, z[i * kWallThreads]);
+    return;
+  }
+  for (int q = threadIdx.x; q < n * pitch; q += kWallThreads) {
+    const int j = q / pitch, i = q - j * pitch;
+    Mt[q] = i < n ? M[i * n + j] : 0.0f;
+  }
+  __syncthreads();
+  if (!in) return;
+  for (int i = 0; i < n; i += kWallRows) {
+    float2 acc[kWallRows];
+#pragma unroll
+    for (int r = 0; r < kWallRows; ++r) acc[r] = make_float2(0.f, 0.f);
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+      const float2 v = z[j * kWallThreads];
+      float m[kWallRows];
+      const float4* row = reinterpret_cast<const float4*>(Mt + j * pitch + i);
+      *reinterpret_cast<float4*>(m) = row[0];
+      *reinterpret_cast<float4*>(m + 4) = row[1];
+#pragma unroll
+      for (int r = 0; r < kWallRows; ++r) {
+        acc[r].x += v.x * m[r];
+        acc[r].y += v.y * m[r];
       }
     }
-    if (a.out) a.out[i * a.n_pix + k] = make_float2(acc.re, acc.im);
-    p += cnorm(acc);
+#pragma unroll
+    for (int r = 0; r < kWallRows; ++r)
+      if (i + r < n) store(i + r, acc[r]);
   }
-  if (a.power) a.power[k] = p;
+}
+
+__global__ void __launch_bounds__(kWallThreads) wall_kernel(const WallArgs a) {
+  extern __shared__ float4 wall_s[];
+  const long k = blockIdx.x * static_cast<long>(kWallThreads) + threadIdx.x;
+  float p = 0.0f;
+  wall_pixel(wall_s, a.ens + k, a.n_pix, a.n, a.M, a.identity, k < a.n_pix, [&](int i, float2 v) {
+    if (a.out) a.out[i * a.n_pix + k] = v;
+    p += cnorm(mk(v.x, v.y));
+  });
+  if (a.power && k < a.n_pix) a.power[k] = p;
 }
 
 struct FlowArgs {
@@ -97,6 +140,40 @@ struct FlowArgs {
   uint8_t* valid;
   unsigned* pmax_bits;
 };
+
+// Velocity, power, variance and the coherence gate of one pixel from its sums.
+__device__ __forceinline__ void flow_finish(const FlowArgs& a, long k, float R00, cplx R01, cplx R10) {
+  float vel = 0.0f, var = 0.0f;
+  uint8_t ok = 0;
+  if (R00 > 0.0f) {
+    const float coherence = cabsf_(R01) / R00;
+    var = fclamp(2.0f * (1.0f - coherence), 0.0f, 1.0f);
+    if (!(coherence < a.coh_thr)) {
+      const float phase_slow = atan2f(R01.im, R01.re);
+      float f_centre = a.fdem;
+      if (a.loupas) {
+        const float phase_fast = atan2f(R10.im, R10.re);
+        const float f_est = phase_fast * a.c / (4.0f * kPi * a.dz);
+        if (f_est > 0.25f * a.fdem && f_est < 2.0f * a.fdem) f_centre = f_est;
+      }
+      if (f_centre > 0.0f) {
+        vel = -phase_slow * a.c * a.prf / (4.0f * kPi * f_centre);
+        ok = 1;
+      }
+    }
+  }
+  a.velocity[k] = vel;
+  a.power[k] = R00;
+  a.variance[k] = var;
+  a.valid[k] = ok;
+}
+
+// The warp's largest power into the frame's maximum (every lane calls it;
+// power is non-negative, so its bit pattern orders like its value).
+__device__ __forceinline__ void flow_peak(const FlowArgs& a, float power) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(power, 0.0f)));
+  if ((threadIdx.x & 31) == 0) atomicMax(a.pmax_bits, m);
+}
 
 __device__ __forceinline__ void flow_pixel(const FlowArgs& a) {
   const long k0 = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
@@ -130,38 +207,103 @@ __device__ __forceinline__ void flow_pixel(const FlowArgs& a) {
       }
     }
   }
-  float vel = 0.0f, var = 0.0f;
-  uint8_t ok = 0;
-  if (R00 > 0.0f) {
-    const float coherence = cabsf_(R01) / R00;
-    var = fclamp(2.0f * (1.0f - coherence), 0.0f, 1.0f);
-    if (!(coherence < a.coh_thr)) {
-      const float phase_slow = atan2f(R01.im, R01.re);
-      float f_centre = a.fdem;
-      if (a.loupas) {
-        const float phase_fast = atan2f(R10.im, R10.re);
-        const float f_est = phase_fast * a.c / (4.0f * kPi * a.dz);
-        if (f_est > 0.25f * a.fdem && f_est < 2.0f * a.fdem) f_centre = f_est;
+  if (in_range) flow_finish(a, k, R00, R01, R10);
+  flow_peak(a, R00);
+}
+
+constexpr int kFlowCols = 128;   // depths per block of the line kernels
+
+// The same sums for kFlowLines lateral lines per thread, a block of kFlowCols
+// depths. An output's sums run over its window in (line, depth, frame) order,
+// so a product z_e^* z_e+1 formed once for (line, depth, frame) can be added to
+// each of the thread's outputs (up to 2 kKL + 1) whose window holds that line,
+// and every output still adds its terms in that order: the maps equal
+// flow_pixel's bit for bit. The block's lines pass through shared memory one
+// at a time, all frames of each ([frame][depth], halo included, zeros outside
+// the grid), because the frames are the innermost loop: read through L1, the
+// frames of a line are evicted before the next depth of the window reads them
+// again (413 us).
+// What bounds it: dependent issue at 24 warps per SM (35 KB of shared memory
+// per block at 32 frames). 8 ensembles of 8 to 32 frames, 256 x 512, 9 x 3
+// windows: 333 us, flow_kernel's pixel per thread 469; 13 x 5 windows: 590
+// against 1,080. Eight lines: 306 and 550, but half the threads (one ensemble
+// of 32 frames 142 us against 108). The open outputs in a rolling set of
+// registers, any number of lines: 394 to 556. A branch without the last
+// depth's selects doubles the unrolled code: 358.
+constexpr int kFlowLines = 4;
+template <int kKL>
+__device__ __forceinline__ void flow_lines(const FlowArgs& a) {
+  extern __shared__ float2 fl_s[];   // [n][kFlowCols + 2 ka + 1]
+  const long n_pix = static_cast<long>(a.n0) * a.n1;
+  const int width = kFlowCols + 2 * a.ka + 1;
+  const int i0 = blockIdx.y * kFlowLines, j0 = blockIdx.x * kFlowCols;
+  const int j = j0 + threadIdx.x;
+  float2 R01[kFlowLines], R10[kFlowLines];
+  float R00[kFlowLines];
+#pragma unroll
+  for (int r = 0; r < kFlowLines; ++r) {
+    R01[r] = R10[r] = make_float2(0.f, 0.f);
+    R00[r] = 0.0f;
+  }
+#pragma unroll
+  for (int q = 0; q < kFlowLines + 2 * kKL; ++q) {   // line i0 - kKL + q
+    const int ii = i0 - kKL + q;
+    if (ii < 0 || ii >= a.n0) continue;
+    __syncthreads();   // the previous line is no longer read
+    const float2* line = a.filt + static_cast<long>(ii) * a.n1;
+    for (int c = threadIdx.x; c < width; c += kFlowCols) {
+      const int jj = j0 - a.ka + c;
+      const bool in = jj >= 0 && jj < a.n1;
+#pragma unroll 8
+      for (int e = 0; e < a.n; ++e) fl_s[e * width + c] = in ? __ldg(line + e * n_pix + jj) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    for (int d = 0; d <= 2 * a.ka; ++d) {
+      // z is zero outside the grid; the last depth has no next one.
+      const int jj = j - a.ka + d;
+      const bool next = jj >= 0 && jj + 1 < a.n1;
+      const float2* p = fl_s + threadIdx.x + d;
+      float2 z = *p;
+      auto add = [&](float2 zc, float2 zn, float2 w, bool last) {
+        const float zz = zc.x * zc.x + zc.y * zc.y;
+        const float2 zr = next ? zc : make_float2(0.f, 0.f);
+        const float2 wr = next ? w : make_float2(0.f, 0.f);
+        const float2 fast = make_float2(zr.x * wr.x + zr.y * wr.y, zr.x * wr.y - zr.y * wr.x);
+        float2 slow = make_float2(0.f, 0.f);
+        if (!last) slow = make_float2(zc.x * zn.x + zc.y * zn.y, zc.x * zn.y - zc.y * zn.x);
+#pragma unroll
+        for (int r = 0; r < kFlowLines; ++r) {
+          if (q < r || q > r + 2 * kKL) continue;   // the line is outside output r's window
+          R00[r] += zz;
+          if (!last) R01[r] = __fadd2_rn(R01[r], slow);
+          R10[r] = __fadd2_rn(R10[r], fast);
+        }
+      };
+#pragma unroll 4
+      for (int e = 0; e + 1 < a.n; ++e) {
+        const float2 zn = p[(e + 1) * width];
+        add(z, zn, p[e * width + 1], false);
+        z = zn;
       }
-      if (f_centre > 0.0f) {
-        vel = -phase_slow * a.c * a.prf / (4.0f * kPi * f_centre);
-        ok = 1;
-      }
+      add(z, z, p[(a.n - 1) * width + 1], true);
     }
   }
-  if (in_range) {
-    a.velocity[k] = vel;
-    a.power[k] = R00;
-    a.variance[k] = var;
-    a.valid[k] = ok;
+  float peak = 0.0f;
+#pragma unroll
+  for (int r = 0; r < kFlowLines; ++r) {
+    const int i = i0 + r;
+    if (i >= a.n0 || j >= a.n1) continue;
+    flow_finish(a, static_cast<long>(i) * a.n1 + j, R00[r], mk(R01[r].x, R01[r].y), mk(R10[r].x, R10[r].y));
+    peak = fmaxf(peak, R00[r]);
   }
-  // Power is non-negative, so its bit pattern orders like its value.
-  unsigned m = __float_as_uint(fmaxf(R00, 0.0f));
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(a.pmax_bits, m);
+  flow_peak(a, peak);
 }
 
 __global__ void flow_kernel(const FlowArgs a) { flow_pixel(a); }
+template <int kKL>
+__global__ void __launch_bounds__(kFlowCols) flow_lines_kernel(const FlowArgs a) {
+  flow_lines<kKL>(a);
+}
 
 __global__ void power_gate_kernel(const float* power, uint8_t* valid, long n, float ratio,
                                   const unsigned* pmax_bits) {
@@ -196,30 +338,14 @@ struct WallBatchArgs {
   float M[kBatchPool];
 };
 
-__global__ void wall_batch_kernel(const WallBatchArgs a) {
-  extern __shared__ float2 zs[];   // [n][blockDim]
+__global__ void __launch_bounds__(kWallThreads) wall_batch_kernel(const WallBatchArgs a) {
+  extern __shared__ float4 wall_s[];
   const int e = blockIdx.y;
-  const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
-  if (k >= a.n_pix) return;
-  const int n = a.n[e];
+  const long k = blockIdx.x * static_cast<long>(kWallThreads) + threadIdx.x;
   const float2* src = a.ens + a.in_off[e] * a.n_pix;
   float2* dst = a.out + a.out_off[e] * a.n_pix;
-  const float* M = a.M + a.m_off[e];
-  for (int j = 0; j < n; ++j) zs[j * blockDim.x + threadIdx.x] = src[j * a.n_pix + k];
-  for (int i = 0; i < n; ++i) {
-    cplx acc;
-    if (a.identity) {
-      const float2 z = zs[i * blockDim.x + threadIdx.x];
-      acc = mk(z.x, z.y);
-    } else {
-      acc = mk(0.f, 0.f);
-      for (int j = 0; j < n; ++j) {
-        const float2 z = zs[j * blockDim.x + threadIdx.x];
-        acc = cadd(acc, cscale(mk(z.x, z.y), M[i * n + j]));
-      }
-    }
-    dst[i * a.n_pix + k] = make_float2(acc.re, acc.im);
-  }
+  wall_pixel(wall_s, src + k, a.n_pix, a.n[e], a.M + a.m_off[e], a.identity, k < a.n_pix,
+             [&](int i, float2 v) { dst[i * a.n_pix + k] = v; });
 }
 
 struct FlowBatchArgs {
@@ -229,8 +355,8 @@ struct FlowBatchArgs {
   long f_off[kBatchEns];
 };
 
-__global__ void flow_batch_kernel(const FlowBatchArgs b) {
-  const int e = blockIdx.y;
+// Entry e of the chunk as one ensemble's arguments.
+__device__ __forceinline__ FlowArgs flow_entry(const FlowBatchArgs& b, int e) {
   FlowArgs a = b.base;
   const long n_pix = static_cast<long>(a.n0) * a.n1;
   const long row = b.ens[e];
@@ -241,7 +367,12 @@ __global__ void flow_batch_kernel(const FlowBatchArgs b) {
   a.variance += row * n_pix;
   a.valid += row * n_pix;
   a.pmax_bits += row;
-  flow_pixel(a);
+  return a;
+}
+__global__ void flow_batch_kernel(const FlowBatchArgs b) { flow_pixel(flow_entry(b, blockIdx.y)); }
+template <int kKL>
+__global__ void __launch_bounds__(kFlowCols) flow_lines_batch_kernel(const FlowBatchArgs b) {
+  flow_lines<kKL>(flow_entry(b, blockIdx.z));
 }
 
 __global__ void power_gate_batch_kernel(const float* power, uint8_t* valid, long n, float ratio,
@@ -535,8 +666,8 @@ int launch_wall(usx_ctx* ctx, const float* ens, int n, long n_pix, int type, int
     const std::vector<float> M = reject_matrix(n, type == USX_WALL_MEAN ? 0 : order);
     std::copy(M.begin(), M.end(), a.M);
   }
-  const int threads = 128;
-  const size_t smem = sizeof(float2) * n * threads;
+  const int threads = kWallThreads;
+  const size_t smem = wall_smem(n);
   if (smem > 48 * 1024)
     if (int rc_ = smem_limit(reinterpret_cast<const void*>(wall_kernel), static_cast<size_t>(static_cast<int>(smem)))) return rc_;
   prof_begin(ctx, "wall_kernel");
@@ -544,6 +675,40 @@ int launch_wall(usx_ctx* ctx, const float* ens, int n, long n_pix, int type, int
   prof_end(ctx);
   USX_CHECK_LAUNCH("wall_kernel");
   return USX_OK;
+}
+
+// The flow sums of `count` ensembles of at most max_n frames. Four lines per
+// thread where the windows span lines (kl of 1 or 2) and a quarter of the
+// pixels as threads still fills the GPU (wall filter and gate included, us,
+// pixel per thread against four lines; 9 x 3 windows: one ensemble of 32
+// frames, 64 x 256, 65 / 98; 256 x 512, 165 / 143; 8 frames, 50 / 45; two of
+// 4 and 6 frames, 256 x 256, 41 / 51; 13 x 5 windows, 24 frames, 256 x 256:
+// 154 / 116; 9 x 5, 32 frames, 121 x 333: 139 / 119; 5 x 1: 232 / 269).
+bool flow_lines_pay(const FlowArgs& a, int max_n, int count, size_t smem) {
+  const long pixels = static_cast<long>(a.n0) * a.n1 * count;
+  return (a.kl == 1 || a.kl == 2) && max_n >= 8 && pixels >= (a.kl == 1 ? 120000 : 40000) && smem <= 200 * 1024 &&
+         ceil_div(a.n0, kFlowLines) <= 65535;
+}
+template <typename Args, typename Pixel, typename Lines>
+int launch_flow_sums(cudaStream_t st, const FlowArgs& a, const Args& args, int max_n, int count, Pixel pixel,
+                     Lines lines1, Lines lines2) {
+  const size_t smem = sizeof(float2) * static_cast<size_t>(max_n) * (kFlowCols + 2 * static_cast<size_t>(a.ka) + 1);
+  if (!flow_lines_pay(a, max_n, count, smem)) {
+    pixel<<<dim3(ceil_div(static_cast<long>(a.n0) * a.n1, 128), count), 128, 0, st>>>(args);
+    return USX_OK;
+  }
+  Lines kern = a.kl == 1 ? lines1 : lines2;
+  if (smem > 48 * 1024)
+    if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), smem)) return rc_;
+  kern<<<dim3(ceil_div(a.n1, kFlowCols), ceil_div(a.n0, kFlowLines), count), kFlowCols, smem, st>>>(args);
+  return USX_OK;
+}
+int launch_flow_sums(cudaStream_t st, const FlowArgs& a) {
+  return launch_flow_sums(st, a, a, a.n, 1, flow_kernel, flow_lines_kernel<1>, flow_lines_kernel<2>);
+}
+int launch_flow_sums(cudaStream_t st, const FlowBatchArgs& b, int max_n, int count) {
+  return launch_flow_sums(st, b.base, b, max_n, count, flow_batch_kernel, flow_lines_batch_kernel<1>,
+                          flow_lines_batch_kernel<2>);
 }
 
 int launch_flow(usx_ctx* ctx, const float* filt, int n, int n0, int n1, float dz, float fdem,
@@ -570,7 +735,7 @@ int launch_flow(usx_ctx* ctx, const float* filt, int n, int n0, int n1, float dz
   const long n_pix = static_cast<long>(n0) * n1;
   USX_CUDA(cudaMemsetAsync(pmax_bits, 0, sizeof(unsigned), ctx->stream));
   prof_begin(ctx, "flow_kernel");
-  flow_kernel<<<ceil_div(n_pix, 128), 128, 0, ctx->stream>>>(a);
+  if (int rc = launch_flow_sums(ctx->stream, a)) return rc;
   prof_end(ctx);
   USX_CHECK_LAUNCH("flow_kernel");
   const float ratio = std::pow(10.0f, cfg.power_threshold_db / 10.0f);
@@ -695,7 +860,7 @@ int usx_cu_color_flow_batch(usx_ctx* ctx, const float* ens, int n_ens, const int
 
   const int type = cfg->wall_filter;
   const int order = type == USX_WALL_MEAN ? 0 : cfg->polynomial_order;
-  const int threads = 128;
+  const int threads = kWallThreads;
   FlowBatchArgs fb;
   FlowArgs& f = fb.base;
   f.filt = filt;
@@ -754,7 +919,7 @@ int usx_cu_color_flow_batch(usx_ctx* ctx, const float* ens, int n_ens, const int
       chunk_max = std::max(chunk_max, n);
       ++count;
     }
-    const size_t smem = sizeof(float2) * static_cast<size_t>(chunk_max) * threads;
+    const size_t smem = wall_smem(chunk_max);
     if (smem > 48 * 1024)
       if (int rc_ = smem_limit(reinterpret_cast<const void*>(wall_batch_kernel), smem)) return rc_;
     prof_begin(ctx, "wall_batch_kernel");
@@ -762,7 +927,7 @@ int usx_cu_color_flow_batch(usx_ctx* ctx, const float* ens, int n_ens, const int
     prof_end(ctx);
     USX_CHECK_LAUNCH("wall_batch_kernel");
     prof_begin(ctx, "flow_batch_kernel");
-    flow_batch_kernel<<<dim3(ceil_div(n_pix, 128), count), 128, 0, ctx->stream>>>(fb);
+    if (int rc = launch_flow_sums(ctx->stream, fb, chunk_max, count)) return rc;
     prof_end(ctx);
     USX_CHECK_LAUNCH("flow_batch_kernel");
     e0 += count;
@@ -807,8 +972,8 @@ int usx_cu_color_flow_noalloc(void* stream, const float* ens, int n_frames, int 
     const std::vector<float> M = reject_matrix(n_frames, cfg->wall_filter == USX_WALL_MEAN ? 0 : cfg->polynomial_order);
     std::copy(M.begin(), M.end(), w.M);
   }
-  const int threads = 128;
-  const size_t smem = sizeof(float2) * n_frames * threads;
+  const int threads = kWallThreads;
+  const size_t smem = wall_smem(n_frames);
   if (smem > 48 * 1024)
     if (int rc_ = smem_limit(reinterpret_cast<const void*>(wall_kernel), static_cast<size_t>(static_cast<int>(smem)))) return rc_;
   wall_kernel<<<ceil_div(n_pix, threads), threads, smem, st>>>(w);
@@ -834,7 +999,7 @@ int usx_cu_color_flow_noalloc(void* stream, const float* ens, int n_frames, int 
   f.pmax_bits = pmax_bits;
   // The scratch keeps the previous call's contents: the running maximum must start at zero.
   USX_CUDA(cudaMemsetAsync(pmax_bits, 0, sizeof(unsigned), st));
-  flow_kernel<<<ceil_div(n_pix, 128), 128, 0, st>>>(f);
+  if (int rc = launch_flow_sums(st, f)) return rc;
   USX_CHECK_LAUNCH("flow_kernel");
   const float ratio = std::pow(10.0f, cfg->power_threshold_db / 10.0f);
   power_gate_kernel<<<ceil_div(n_pix, 256), 256, 0, st>>>(power, valid, n_pix, ratio, pmax_bits);
