@@ -27,6 +27,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "tc5.cuh"
 #include "usx_internal.cuh"
@@ -1190,6 +1191,401 @@ __global__ void __launch_bounds__(32 * kWarpMvWarps) mv_warp_kernel(const MvWarp
 }
 
 // ---------------------------------------------------------------------------
+// The FP32 minimum variance (USX_MV_FP32), one warp per pixel
+// (mv_fp32_kernel<kPan>): the covariance by diagonals, a blocked Cholesky
+// factorisation R + eps I = F F^H, and the output from the factor alone. With
+// y = F^-1 1 and z = F^-1 a (a the centre row's subarray average),
+//     sum w = 1^H R^-1 1 = |y|^2,   w^H a = 1^H R^-1 a = y^H z,
+// so w itself is not formed and neither substitution is run: 1^H and a^H ride
+// along as two more rows of the factorisation (row L becomes y^H, row L + 1
+// z^H). The training export needs w and keeps mv_warp_kernel.
+//
+// Covariance: with G_m(t) = sum_d x_d[t + m] conj(x_d[t]), the first entry of
+// diagonal m is the sum of G_m(t) over t < n_sub, and each further one follows
+// as R[i + 1][k + 1] = R[i][k] - G_m(k) + G_m(n_sub + k). The G_m(k) taken off
+// were formed for the first sum (n_sub > L): they wait in the entries they
+// lead to.
+//
+// Factorisation: panels of four columns. A lane holds the panel entries of
+// rows c0 + lane + 32 s in registers (pivots and multipliers by shuffles),
+// leaves the panel in shared memory as (re, re, im, im) quadruples, and
+// updates its own rows of the trailing triangle by rank 4 in FP32 pairs.
+//
+// 128 channels, 75 plane waves, 512 x 1024 pixels, L up to 64: 9.5 ms against
+// 15.5 for mv_warp_kernel (staging 2.3, covariance with both products of every
+// step 3.4, factor with its panels in shared memory 5.7, substitutions 4.1). What
+// bounds it: the shared-memory pipe for L of 17 to 48 (75% of its wavefronts,
+// the trailing rows' reads and writes), latency at 10 warps per SM for L up to
+// 64 (22 KB of shared memory per pixel).
+constexpr int kMvPanel = 4;
+// Warps per CTA: the warps are independent, and small CTAs fit more of them
+// beside one another in shared memory (1, 2 and 4 warps: 3.54, 3.56, 4.07 ms
+// for the class of L up to 64; 1.77, 1.69, 1.67 for L up to 32).
+constexpr int kMvFp32Warps = 2;
+
+struct MvFp32Layout {
+  size_t off_act, off_x, off_r, bytes;   // per warp
+  int pitch;                             // row pitch of the staged rows (even)
+};
+// The staged rows, once the covariance and the centre row's average are formed,
+// give their space to the panel (kMvPanel quadruples per row) and the two
+// right-hand rows.
+__host__ __device__ inline MvFp32Layout mv_fp32_layout(int nmax, int n_dmax, int lmax) {
+  MvFp32Layout l;
+  l.pitch = (nmax + 1) & ~1;
+  size_t o = 0;
+  l.off_act = o; o = align16(o + sizeof(int) * nmax);
+  const size_t rows = sizeof(float2) * n_dmax * l.pitch;
+  const size_t panel = (sizeof(float4) * kMvPanel + 2 * sizeof(float2)) * static_cast<size_t>(lmax);
+  l.off_x = o;   o = align16(o + (rows > panel ? rows : panel));
+  l.off_r = o;   o = align16(o + sizeof(float2) * (lmax * (lmax + 1) / 2));
+  l.bytes = o;
+  return l;
+}
+
+__device__ __forceinline__ float2 shfl2(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// Factors the packed lower triangle Rl (L rows) with the two right-hand rows
+// Rx[0..L) and Rx[lx..lx + L), which become F^-1's (see above). P: L x kMvPanel
+// quadruples. False on a non-positive pivot.
+template <int kPan>
+__device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, float4* P, int L, int lane) {
+  for (int c0 = 0; c0 < L; c0 += kMvPanel) {
+    const int nb = min(kMvPanel, L - c0);
+    float2 v[kPan][kMvPanel];
+    float2* row[kPan];
+#pragma unroll
+    for (int s = 0; s < kPan; ++s) {
+      const int i = c0 + lane + 32 * s;
+      row[s] = i < L ? Rl + tri(i, 0) : Rx + (i == L ? 0 : lx);
+#pragma unroll
+      for (int c = 0; c < kMvPanel; ++c)
+        v[s][c] = c < nb && i < L + 2 && (s > 0 || lane >= c) ? row[s][c0 + c] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int c = 0; c < kMvPanel; ++c) {
+      if (c >= nb) break;
+      const float d = __shfl_sync(0xffffffffu, v[0][c].x, c);
+      if (!(d > 0.0f)) return false;
+      float inv = rsqrtf(d);
+      inv = inv * fmaf(-0.5f * d * inv, inv, 1.5f);
+#pragma unroll
+      for (int s = 0; s < kPan; ++s) v[s][c] = make_float2(v[s][c].x * inv, v[s][c].y * inv);
+#pragma unroll
+      for (int cc = c + 1; cc < kMvPanel; ++cc) {
+        if (cc >= nb) break;
+        const float2 m = shfl2(v[0][c], cc);
+#pragma unroll
+        for (int s = 0; s < kPan; ++s) {
+          v[s][cc].x = fmaf(-v[s][c].x, m.x, fmaf(-v[s][c].y, m.y, v[s][cc].x));
+          v[s][cc].y = fmaf(-v[s][c].y, m.x, fmaf(v[s][c].x, m.y, v[s][cc].y));
+        }
+      }
+    }
+    const int k0 = c0 + nb;
+#pragma unroll
+    for (int s = 0; s < kPan; ++s) {
+      const int i = c0 + lane + 32 * s;
+      if (i < k0 || i >= L + 2) continue;
+      if (i < L) {
+#pragma unroll
+        for (int c = 0; c < kMvPanel; ++c) P[kMvPanel * i + c] = make_float4(v[s][c].x, v[s][c].x, v[s][c].y, v[s][c].y);
+      } else {
+#pragma unroll
+        for (int c = 0; c < kMvPanel; ++c)
+          if (c < nb) row[s][c0 + c] = v[s][c];
+      }
+    }
+    __syncwarp();
+    if (k0 >= L) break;
+    // Trailing rows: R[i][k] -= sum_c v_ic conj(v_kc), k0 <= k <= min(i, L - 1).
+    float2 f1[kPan][kMvPanel], f2[kPan][kMvPanel];
+    int last[kPan];
+#pragma unroll
+    for (int s = 0; s < kPan; ++s) {
+      const int i = c0 + lane + 32 * s;
+      last[s] = i >= k0 && i < L + 2 ? min(i, L - 1) : -1;
+#pragma unroll
+      for (int c = 0; c < kMvPanel; ++c) {
+        f1[s][c] = make_float2(-v[s][c].x, -v[s][c].y);
+        f2[s][c] = make_float2(-v[s][c].y, v[s][c].x);
+      }
+    }
+    auto update = [&](auto from, int k_lo, int k_hi) {
+      constexpr int S0 = decltype(from)::value;   // the slots below are done
+#pragma unroll 2
+      for (int k = k_lo; k <= k_hi; ++k) {
+        float4 p[kMvPanel];
+#pragma unroll
+        for (int c = 0; c < kMvPanel; ++c) p[c] = P[kMvPanel * k + c];
+#pragma unroll
+        for (int s = S0; s < kPan; ++s) {
+          if (k > last[s]) continue;
+          float2 r = row[s][k];
+#pragma unroll
+          for (int c = 0; c < kMvPanel; ++c) {
+            r = __ffma2_rn(f1[s][c], make_float2(p[c].x, p[c].y), r);
+            r = __ffma2_rn(f2[s][c], make_float2(p[c].z, p[c].w), r);
+          }
+          row[s][k] = r;
+        }
+      }
+    };
+    update(std::integral_constant<int, 0>{}, k0, min(L - 1, c0 + 31));
+    if constexpr (kPan > 1) update(std::integral_constant<int, 1>{}, max(k0, c0 + 32), L - 1);
+    __syncwarp();
+  }
+  return true;
+}
+
+template <int kPan>
+__global__ void __launch_bounds__(32 * kMvFp32Warps) mv_fp32_kernel(const MvWarpArgs wa) {
+  extern __shared__ float4 mvw_smem_raw[];
+  const MvTcArgs& a = wa.base;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  const MvFp32Layout lay = mv_fp32_layout(wa.nmax, a.n_dmax, wa.lmax);
+  char* base = reinterpret_cast<char*>(mvw_smem_raw) + warp * lay.bytes;
+  int* act = reinterpret_cast<int*>(base + lay.off_act);
+  float2* x = reinterpret_cast<float2*>(base + lay.off_x);
+  float2* Rl = reinterpret_cast<float2*>(base + lay.off_r);
+  float4* P = reinterpret_cast<float4*>(x);
+  float2* Rx = reinterpret_cast<float2*>(P + kMvPanel * wa.lmax);
+  const int nmax = wa.nmax, pitch = lay.pitch;
+
+  const long n_items = wa.pair_list ? static_cast<long>(min(*wa.pair_count, wa.pair_cap))
+                                    : static_cast<long>(wa.n_list) * wa.n_frames;
+  for (long item = static_cast<long>(blockIdx.x) * n_warps + warp; item < n_items;
+       item += static_cast<long>(gridDim.x) * n_warps) {
+    int pix;
+    long frame;
+    if (wa.pair_list) {
+      const int2 pf = wa.pair_list[item];
+      pix = pf.x;
+      frame = pf.y;
+    } else {
+      frame = item / wa.n_list;
+      pix = wa.pix_list[item - frame * wa.n_list];
+    }
+    const int j = pix % a.n1;
+    const float px = __ldg(a.points + 3 * pix), pz = __ldg(a.points + 3 * pix + 2);
+    const float2* Y = a.y + frame * static_cast<long>(a.n_pix) * a.n_ch;
+    __syncwarp();
+    int n_act = 0;
+    for (int c0 = 0; c0 < a.n_ch; c0 += 32) {
+      const int ch = c0 + lane;
+      bool on = false;
+      if (ch < a.n_ch)
+        on = aperture_weight((static_cast<float>(ch) - a.half_nm1) * a.pitch, px, pz, a.f_number, a.rx_window,
+                             a.tukey_alpha) > 0.0f;
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      if (on && n_act + __popc(m & ((1u << lane) - 1u)) < nmax) act[n_act + __popc(m & ((1u << lane) - 1u))] = ch;
+      n_act += __popc(m);
+    }
+    __syncwarp();
+    auto finish = [&](cplx out, float cre, float cim, float inc) {  // lane 0
+      if (a.cf && n_act > 0) {
+        const float coh = cre * cre + cim * cim;
+        out = cscale(out, (inc > 0.0f) ? coh / (static_cast<float>(n_act) * inc) : 0.0f);
+      }
+      if (a.incoherent)
+        a.acc_out[frame * a.n_pix + pix] += cnorm(out);
+      else
+        a.out[frame * a.out_stride + pix] = make_float2(out.re, out.im);
+    };
+    int L = a.mv_subarray;
+    const int hi = max(2, n_act / 2);
+    if (L < 2) L = 2;
+    if (L > hi) L = hi;
+    if (n_act > nmax || L > wa.lmax) {
+      if (lane == 0 && wa.overflow_count) {
+        const int slot = atomicAdd(wa.overflow_count, 1);
+        if (slot < wa.overflow_cap) wa.overflow[slot] = make_int2(pix, static_cast<int>(frame));
+      }
+      continue;
+    }
+    const float2* yc = Y + static_cast<long>(pix) * a.n_ch;
+    if (n_act < 4) {
+      if (lane == 0) {
+        // The reference's rule: the DAS sum, channels in ascending order.
+        cplx acc = mk(0.f, 0.f);
+        float inc = 0.0f;
+        for (int q = 0; q < n_act; ++q) {
+          const float2 v = yc[act[q]];
+          acc = cadd(acc, mk(v.x, v.y));
+          inc += cnorm(mk(v.x, v.y));
+        }
+        if (n_act == 0) {
+          if (!a.incoherent) a.out[frame * a.out_stride + pix] = make_float2(0.f, 0.f);
+        } else {
+          finish(acc, acc.re, acc.im, inc);
+        }
+      }
+      continue;
+    }
+    const int n_sub = n_act - L + 1;
+    int dlo = -a.range_avg, dhi = a.range_avg;
+    while (j + dlo < 0) ++dlo;
+    while (j + dhi >= a.n1) --dhi;
+    const int n_d = dhi - dlo + 1, dc = -dlo;
+
+    // FP32 rows of the active channels, largest magnitude.
+    float amax = 0.0f;
+    {
+      const float2* y0 = Y + static_cast<long>(pix + dlo) * a.n_ch;
+#pragma unroll 2
+      for (int q = lane; q < n_act; q += 32) {
+        const float2* src = y0 + act[q];
+#pragma unroll 5
+        for (int d = 0; d < n_d; ++d) {
+          const float2 v = src[static_cast<long>(d) * a.n_ch];
+          x[d * pitch + q] = v;
+          amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
+        }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    __syncwarp();
+    // Coherence-factor terms of the centre row.
+    float cre = 0.f, cim = 0.f, inc = 0.f;
+    if (a.cf) {
+      for (int q = lane; q < n_act; q += 32) {
+        const float2 v = x[dc * pitch + q];
+        cre += v.x;
+        cim += v.y;
+        inc += v.x * v.x + v.y * v.y;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        cre += __shfl_xor_sync(0xffffffffu, cre, o);
+        cim += __shfl_xor_sync(0xffffffffu, cim, o);
+        inc += __shfl_xor_sync(0xffffffffu, inc, o);
+      }
+    }
+    if (!(amax > 0.0f)) {
+      if (lane == 0) finish(mk(0.f, 0.f), cre, cim, inc);
+      continue;
+    }
+    int e2;
+    frexpf(amax, &e2);
+    // Scaled by the power of two 2^-2e2 and by 1 / K.
+    const float f = ldexpf(1.0f, -2 * e2) / static_cast<float>(n_d * n_sub);
+    float tr = 0.0f;   // of the diagonal (lane 0)
+    auto diagonals = [&](auto rows_c) {
+      constexpr int ND = decltype(rows_c)::value;   // rows at compile time, or 0
+      const int nd = ND > 0 ? ND : n_d;
+#pragma unroll 1
+      for (int h = 0; h < (kPan > 1 ? 2 : 1); ++h) {
+        const int m = h == 0 ? lane : 63 - lane;   // lag
+        if (m >= L || (h == 1 && m < 32)) continue;
+        auto G = [&](int t) {
+          float re = 0.f, im = 0.f;
+#pragma unroll
+          for (int d = 0; d < (ND > 0 ? ND : 1); ++d) {
+            const float2 p = x[d * pitch + t + m], q = x[d * pitch + t];
+            re = fmaf(p.x, q.x, fmaf(p.y, q.y, re));
+            im = fmaf(p.y, q.x, fmaf(-p.x, q.y, im));
+          }
+          if (ND == 0)
+            for (int d = 1; d < nd; ++d) {
+              const float2 p = x[d * pitch + t + m], q = x[d * pitch + t];
+              re = fmaf(p.x, q.x, fmaf(p.y, q.y, re));
+              im = fmaf(p.y, q.x, fmaf(-p.x, q.y, im));
+            }
+          return make_float2(re, im);
+        };
+        float2 acc = make_float2(0.f, 0.f);
+        int e = tri(m, 0);   // packed index of entry (m + k, k)
+        int at = e;
+        int t = 0;
+#pragma unroll 2
+        for (; t + 1 + m < L; ++t) {
+          const float2 g = G(t);
+          acc = make_float2(acc.x + g.x, acc.y + g.y);
+          at += m + t + 2;   // tri(i + 1, k + 1) - tri(i, k) = i + 2, i = m + t
+          Rl[at] = g;
+        }
+#pragma unroll 2
+        for (; t < n_sub; ++t) {
+          const float2 g = G(t);
+          acc = make_float2(acc.x + g.x, acc.y + g.y);
+        }
+        Rl[e] = make_float2(acc.x * f, acc.y * f);
+        float sum = acc.x * f;
+#pragma unroll 2
+        for (int k = 0; k + 1 + m < L; ++k) {
+          e += m + k + 2;
+          const float2 out = Rl[e], in = G(n_sub + k);
+          acc = make_float2(acc.x + (in.x - out.x), acc.y + (in.y - out.y));
+          Rl[e] = make_float2(acc.x * f, acc.y * f);
+          sum += acc.x * f;
+        }
+        if (m == 0) tr = sum;
+      }
+    };
+    if (n_d == 5)
+      diagonals(std::integral_constant<int, 5>{});
+    else
+      diagonals(std::integral_constant<int, 0>{});
+    tr = __shfl_sync(0xffffffffu, tr, 0);
+    // The centre row's subarray average.
+    float2 avg[2];
+    const float inv_nsub = 1.0f / static_cast<float>(n_sub);
+#pragma unroll
+    for (int s2 = 0; s2 < 2; ++s2) {
+      const int i = lane + 32 * s2;
+      float are = 0.f, aim = 0.f;
+      if (i < L) {
+        const float2* yr = x + dc * pitch + i;
+#pragma unroll 4
+        for (int s = 0; s < n_sub; ++s) {
+          are += yr[s].x;
+          aim += yr[s].y;
+        }
+      }
+      avg[s2] = make_float2(are * inv_nsub, aim * inv_nsub);
+    }
+    __syncwarp();   // the rows are read for the last time
+    const float eps = fmaxf(a.loading * tr / static_cast<float>(L), 1e-20f);
+#pragma unroll
+    for (int s2 = 0; s2 < 2; ++s2) {
+      const int i = lane + 32 * s2;
+      if (i >= L) continue;
+      Rl[tri(i, i)].x += eps;
+      Rx[i] = make_float2(1.0f, 0.0f);
+      Rx[wa.lmax + i] = make_float2(avg[s2].x, -avg[s2].y);
+    }
+    __syncwarp();
+    const bool ok = chol_augmented<kPan>(Rl, Rx, wa.lmax, P, L, lane);
+    float den = 0.f, nre = 0.f, nim = 0.f;
+    if (ok) {
+      for (int c = lane; c < L; c += 32) {
+        const float2 y = Rx[c], z = Rx[wa.lmax + c];   // conj(y_c), conj(z_c)
+        den = fmaf(y.x, y.x, fmaf(y.y, y.y, den));
+        nre = fmaf(y.x, z.x, fmaf(y.y, z.y, nre));     // conj(y) z
+        nim = fmaf(y.y, z.x, fmaf(-y.x, z.y, nim));
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        den += __shfl_xor_sync(0xffffffffu, den, o);
+        nre += __shfl_xor_sync(0xffffffffu, nre, o);
+        nim += __shfl_xor_sync(0xffffffffu, nim, o);
+      }
+    }
+    if (lane == 0) {
+      cplx out = mk(0.f, 0.f);
+      if (!ok || den < 1e-30f) {
+        if (!ok && a.stats) atomicAdd(a.stats + 1, 1);
+        for (int q = 0; q < n_act; ++q) out = cadd(out, mk(yc[act[q]].x, yc[act[q]].y));
+      } else {
+        const float s = static_cast<float>(n_act) / den;
+        out = mk(nre * s, nim * s);
+      }
+      finish(out, cre, cim, inc);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // The covariance stage on the fifth-generation tensor cores
 // (mv_cov_tc5_kernel<P>): every pixel of a class gets its spatially smoothed
 // covariance as one batched Hermitian rank-K update, G = A A^T, where A is the
@@ -1814,7 +2210,30 @@ int launch_mv_tc(usx_ctx* ctx, const float2* y, const float* points, float2* out
     USX_CHECK_LAUNCH("mv_tc_kernel");
     return USX_OK;
   };
+  // The FP32 mode: items < 0, a work list whose length only the device knows.
+  auto launch_fp32 = [&](MvWarpArgs& w, long items, const char* name) -> int {
+    const MvFp32Layout l = mv_fp32_layout(w.nmax, a.n_dmax, w.lmax);
+    void (*kern)(MvWarpArgs) = w.lmax <= 30   ? mv_fp32_kernel<1>
+                               : w.lmax <= 62 ? mv_fp32_kernel<2>
+                                              : mv_fp32_kernel<3>;
+    const int warps = kMvFp32Warps;
+    const size_t smem = l.bytes * warps;
+    if (smem > 227 * 1024) return fail(USX_ERR_UNSUPPORTED, "minimum variance: class too large for shared memory");
+    if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), smem)) return rc_;
+    int per_sm = 0;
+    if (int rc_ = occupancy(reinterpret_cast<const void*>(kern), 32 * warps, smem, &per_sm)) return rc_;
+    const long resident = static_cast<long>(std::max(1, per_sm)) * ctx->sm_count;
+    const long need = (items + warps - 1) / warps;
+    const long blocks = items < 0 ? resident : std::max(1L, std::min(need, resident * 8));
+    prof_begin(ctx, name);
+    kern<<<static_cast<unsigned>(blocks), 32 * warps, smem, ctx->stream>>>(w);
+    prof_end(ctx);
+    USX_CHECK_LAUNCH(name);
+    return USX_OK;
+  };
   auto launch_warp = [&](MvWarpArgs& w, long items, const char* name) -> int {
+    if (extra.cov_engine == 2 && !extra.w_export)
+      return launch_fp32(w, items, extra.list ? "mv_fp32_kernel(list)" : "mv_fp32_kernel");
     w.cov_recur = extra.cov_engine == 2 ? 1 : 0;
     const MvWarpLayout l = mv_warp_layout(w.nmax, a.n_dmax, w.lmax, w.cov_recur != 0);
     const size_t smem = l.bytes * kWarpMvWarps;
