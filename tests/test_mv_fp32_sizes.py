@@ -1,5 +1,5 @@
 """The FP32 minimum variance (factor with the right-hand sides as rows, panels of
-four columns) at every subarray length where a panel, a row slot or a class
+four or eight columns) at every subarray length where a panel, a row slot or a class
 ends, against the kernel in the reference's operation order."""
 
 from __future__ import annotations

@@ -1206,18 +1206,21 @@ __global__ void __launch_bounds__(32 * kWarpMvWarps) mv_warp_kernel(const MvWarp
 // were formed for the first sum (n_sub > L): they wait in the entries they
 // lead to.
 //
-// Factorisation: panels of four columns. A lane holds the panel entries of
-// rows c0 + lane + 32 s in registers (pivots and multipliers by shuffles),
-// leaves the panel in shared memory as (re, re, im, im) quadruples, and
-// updates its own rows of the trailing triangle by rank 4 in FP32 pairs.
+// Factorisation: panels of four or eight columns. A lane holds the panel entries
+// of rows c0 + lane + 32 s in registers (pivots and multipliers by shuffles),
+// leaves the panel in shared memory, and updates its own rows of the trailing
+// triangle by that rank in FP32 pairs.
 //
-// 128 channels, 75 plane waves, 512 x 1024 pixels, L up to 64: 9.5 ms against
+// 128 channels, 75 plane waves, 512 x 1024 pixels, L up to 64: 8.0 ms against
 // 15.5 for mv_warp_kernel (staging 2.3, covariance with both products of every
 // step 3.4, factor with its panels in shared memory 5.7, substitutions 4.1). What
-// bounds it: the shared-memory pipe for L of 17 to 48 (75% of its wavefronts,
-// the trailing rows' reads and writes), latency at 10 warps per SM for L up to
-// 64 (22 KB of shared memory per pixel).
-constexpr int kMvPanel = 4;
+// bounds it: the shared-memory pipe for L of 17 to 48 (the trailing rows' reads
+// and writes; 75% of its wavefronts with panels of four), latency at 10 warps
+// per SM for L up to 64 (22 KB of shared memory per pixel).
+// Panel width: four columns for L up to 32, eight above, where each pass over
+// the trailing rows then does twice the work per read and write (L up to 32:
+// 1.55 ms at 4, 1.79 at 8; up to 48: 3.51 and 3.32; up to 64: 3.34 and 2.76).
+constexpr int mv_panel(int lmax) { return lmax <= 32 ? 4 : 8; }
 // Warps per CTA: the warps are independent, and small CTAs fit more of them
 // beside one another in shared memory (1, 2 and 4 warps: 3.54, 3.56, 4.07 ms
 // for the class of L up to 64; 1.77, 1.69, 1.67 for L up to 32).
@@ -1228,15 +1231,14 @@ struct MvFp32Layout {
   int pitch;                             // row pitch of the staged rows (even)
 };
 // The staged rows, once the covariance and the centre row's average are formed,
-// give their space to the panel (kMvPanel quadruples per row) and the two
-// right-hand rows.
+// give their space to the panel and the two right-hand rows.
 __host__ __device__ inline MvFp32Layout mv_fp32_layout(int nmax, int n_dmax, int lmax) {
   MvFp32Layout l;
   l.pitch = (nmax + 1) & ~1;
   size_t o = 0;
   l.off_act = o; o = align16(o + sizeof(int) * nmax);
   const size_t rows = sizeof(float2) * n_dmax * l.pitch;
-  const size_t panel = (sizeof(float4) * kMvPanel + 2 * sizeof(float2)) * static_cast<size_t>(lmax);
+  const size_t panel = sizeof(float2) * (mv_panel(lmax) + 2) * static_cast<size_t>(lmax);
   l.off_x = o;   o = align16(o + (rows > panel ? rows : panel));
   l.off_r = o;   o = align16(o + sizeof(float2) * (lmax * (lmax + 1) / 2));
   l.bytes = o;
@@ -1248,24 +1250,24 @@ __device__ __forceinline__ float2 shfl2(float2 v, int src) {
 }
 
 // Factors the packed lower triangle Rl (L rows) with the two right-hand rows
-// Rx[0..L) and Rx[lx..lx + L), which become F^-1's (see above). P: L x kMvPanel
-// quadruples. False on a non-positive pivot.
-template <int kPan>
+// Rx[0..L) and Rx[lx..lx + L), which become y^H and z^H (see above). P: the panel,
+// negated, kW complex per row. False on a non-positive pivot.
+template <int kPan, int kW>
 __device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, float4* P, int L, int lane) {
-  for (int c0 = 0; c0 < L; c0 += kMvPanel) {
-    const int nb = min(kMvPanel, L - c0);
-    float2 v[kPan][kMvPanel];
+  for (int c0 = 0; c0 < L; c0 += kW) {
+    const int nb = min(kW, L - c0);
+    float2 v[kPan][kW];
     float2* row[kPan];
 #pragma unroll
     for (int s = 0; s < kPan; ++s) {
       const int i = c0 + lane + 32 * s;
       row[s] = i < L ? Rl + tri(i, 0) : Rx + (i == L ? 0 : lx);
 #pragma unroll
-      for (int c = 0; c < kMvPanel; ++c)
+      for (int c = 0; c < kW; ++c)
         v[s][c] = c < nb && i < L + 2 && (s > 0 || lane >= c) ? row[s][c0 + c] : make_float2(0.f, 0.f);
     }
 #pragma unroll
-    for (int c = 0; c < kMvPanel; ++c) {
+    for (int c = 0; c < kW; ++c) {
       if (c >= nb) break;
       const float d = __shfl_sync(0xffffffffu, v[0][c].x, c);
       if (!(d > 0.0f)) return false;
@@ -1274,7 +1276,7 @@ __device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, f
 #pragma unroll
       for (int s = 0; s < kPan; ++s) v[s][c] = make_float2(v[s][c].x * inv, v[s][c].y * inv);
 #pragma unroll
-      for (int cc = c + 1; cc < kMvPanel; ++cc) {
+      for (int cc = c + 1; cc < kW; ++cc) {
         if (cc >= nb) break;
         const float2 m = shfl2(v[0][c], cc);
 #pragma unroll
@@ -1291,43 +1293,51 @@ __device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, f
       if (i < k0 || i >= L + 2) continue;
       if (i < L) {
 #pragma unroll
-        for (int c = 0; c < kMvPanel; ++c) P[kMvPanel * i + c] = make_float4(v[s][c].x, v[s][c].x, v[s][c].y, v[s][c].y);
+        for (int c = 0; c < kW; c += 2)
+          P[kW / 2 * i + c / 2] = make_float4(-v[s][c].x, -v[s][c].y, -v[s][c + 1].x, -v[s][c + 1].y);
       } else {
 #pragma unroll
-        for (int c = 0; c < kMvPanel; ++c)
+        for (int c = 0; c < kW; ++c)
           if (c < nb) row[s][c0 + c] = v[s][c];
       }
     }
     __syncwarp();
     if (k0 >= L) break;
     // Trailing rows: R[i][k] -= sum_c v_ic conj(v_kc), k0 <= k <= min(i, L - 1).
-    float2 f1[kPan][kMvPanel], f2[kPan][kMvPanel];
+    float2 f2[kPan][kW];   // v times -j
     int last[kPan];
 #pragma unroll
     for (int s = 0; s < kPan; ++s) {
       const int i = c0 + lane + 32 * s;
       last[s] = i >= k0 && i < L + 2 ? min(i, L - 1) : -1;
 #pragma unroll
-      for (int c = 0; c < kMvPanel; ++c) {
-        f1[s][c] = make_float2(-v[s][c].x, -v[s][c].y);
-        f2[s][c] = make_float2(-v[s][c].y, v[s][c].x);
+      for (int c = 0; c < kW; ++c) {
+        f2[s][c] = make_float2(v[s][c].y, -v[s][c].x);
       }
     }
     auto update = [&](auto from, int k_lo, int k_hi) {
       constexpr int S0 = decltype(from)::value;   // the slots below are done
 #pragma unroll 2
       for (int k = k_lo; k <= k_hi; ++k) {
-        float4 p[kMvPanel];
+        // (The pairs are made here: stored as (re, re, im, im) the reads cost
+        // more than the moves, 11.9 against 11.2 ms per frame.)
+        float2 p1[kW], p2[kW];
 #pragma unroll
-        for (int c = 0; c < kMvPanel; ++c) p[c] = P[kMvPanel * k + c];
+        for (int c = 0; c < kW; c += 2) {
+          const float4 p = P[kW / 2 * k + c / 2];
+          p1[c] = make_float2(p.x, p.x);
+          p2[c] = make_float2(p.y, p.y);
+          p1[c + 1] = make_float2(p.z, p.z);
+          p2[c + 1] = make_float2(p.w, p.w);
+        }
 #pragma unroll
         for (int s = S0; s < kPan; ++s) {
           if (k > last[s]) continue;
           float2 r = row[s][k];
 #pragma unroll
-          for (int c = 0; c < kMvPanel; ++c) {
-            r = __ffma2_rn(f1[s][c], make_float2(p[c].x, p[c].y), r);
-            r = __ffma2_rn(f2[s][c], make_float2(p[c].z, p[c].w), r);
+          for (int c = 0; c < kW; ++c) {
+            r = __ffma2_rn(v[s][c], p1[c], r);
+            r = __ffma2_rn(f2[s][c], p2[c], r);
           }
           row[s][k] = r;
         }
@@ -1340,7 +1350,7 @@ __device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, f
   return true;
 }
 
-template <int kPan>
+template <int kPan, int kW>
 __global__ void __launch_bounds__(32 * kMvFp32Warps) mv_fp32_kernel(const MvWarpArgs wa) {
   extern __shared__ float4 mvw_smem_raw[];
   const MvTcArgs& a = wa.base;
@@ -1351,7 +1361,7 @@ __global__ void __launch_bounds__(32 * kMvFp32Warps) mv_fp32_kernel(const MvWarp
   float2* x = reinterpret_cast<float2*>(base + lay.off_x);
   float2* Rl = reinterpret_cast<float2*>(base + lay.off_r);
   float4* P = reinterpret_cast<float4*>(x);
-  float2* Rx = reinterpret_cast<float2*>(P + kMvPanel * wa.lmax);
+  float2* Rx = reinterpret_cast<float2*>(P) + kW * wa.lmax;
   const int nmax = wa.nmax, pitch = lay.pitch;
 
   const long n_items = wa.pair_list ? static_cast<long>(min(*wa.pair_count, wa.pair_cap))
@@ -1556,7 +1566,7 @@ __global__ void __launch_bounds__(32 * kMvFp32Warps) mv_fp32_kernel(const MvWarp
       Rx[wa.lmax + i] = make_float2(avg[s2].x, -avg[s2].y);
     }
     __syncwarp();
-    const bool ok = chol_augmented<kPan>(Rl, Rx, wa.lmax, P, L, lane);
+    const bool ok = chol_augmented<kPan, kW>(Rl, Rx, wa.lmax, P, L, lane);
     float den = 0.f, nre = 0.f, nim = 0.f;
     if (ok) {
       for (int c = lane; c < L; c += 32) {
@@ -2213,9 +2223,11 @@ int launch_mv_tc(usx_ctx* ctx, const float2* y, const float* points, float2* out
   // The FP32 mode: items < 0, a work list whose length only the device knows.
   auto launch_fp32 = [&](MvWarpArgs& w, long items, const char* name) -> int {
     const MvFp32Layout l = mv_fp32_layout(w.nmax, a.n_dmax, w.lmax);
-    void (*kern)(MvWarpArgs) = w.lmax <= 30   ? mv_fp32_kernel<1>
-                               : w.lmax <= 62 ? mv_fp32_kernel<2>
-                                              : mv_fp32_kernel<3>;
+    // Row slots of a lane: L + 2 rows.
+    void (*kern)(MvWarpArgs) = w.lmax <= 30   ? mv_fp32_kernel<1, 4>
+                               : w.lmax <= 32 ? mv_fp32_kernel<2, 4>
+                               : w.lmax <= 62 ? mv_fp32_kernel<2, 8>
+                                              : mv_fp32_kernel<3, 8>;
     const int warps = kMvFp32Warps;
     const size_t smem = l.bytes * warps;
     if (smem > 227 * 1024) return fail(USX_ERR_UNSUPPORTED, "minimum variance: class too large for shared memory");
