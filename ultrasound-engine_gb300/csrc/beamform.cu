@@ -476,11 +476,14 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_fast_kernel(const B
 //   2.58 ms  index and interpolation arithmetic on FP32 pairs, tiles of 4
 //            lines x 8 depths (narrower trace windows: 3.6 -> 2.2 L1
 //            wavefronts per load)
+//   2.50 ms  the receive weights formed once, waiting in shared memory for the
+//            end of the pass (kept in registers: 2.70); what few events gain
+//            most from: 11 events, 256 x 640, 0.208 -> 0.175
 // Shapes (kG, kPW, kCQ, kWL, kTL) at 75 / 11 events, 512 x 1024 / 256 x 640:
-// (4,1,8,4,4) 2.58 / 0.253 ms, (4,2,8,4,8) 2.62 / 0.234, (4,2,4,4,8) 2.80 /
-// 0.219, (4,4,4,4,4) 4.02 / 0.208 (its 75-event table leaves one CTA per SM),
-// (4,2,8,2,2) 2.82 / 0.236, (2,2,8,4,8) 2.74 / 0.225, 8 channels per group
-// 4.5 / 0.319, 40 registers with three CTAs 3.5 / 0.226.
+// (4,1,8,4,4) 2.50 / 0.203 ms, (4,2,8,4,8) 2.55 / 0.201, (4,2,4,4,8) 2.67 /
+// 0.175, (4,4,4,4,4) 3.85 / 0.179 (its 75-event table leaves one CTA per SM).
+// Before the last step: (4,2,8,2,2) 2.82 / 0.236, (2,2,8,4,8) 2.74 / 0.225, 8
+// channels per group 4.5 / 0.319, 40 registers with three CTAs 3.5 / 0.226.
 constexpr int kTabEvents = 80;   // events a CTA tabulates at once (more go in chunks)
 
 // Dynamic shared memory of the channel-warp kernels: the transmit table of
@@ -602,9 +605,12 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
       float r = INFINITY;   // an inactive channel's sample index is past every trace
       if (valid && grp < g_hi && ch < a.n_ch) {
         const float ex = elem_x(a, ch);
-        if (aperture_weight(ex, px, pz, a.f_number, a.rx_window, a.tukey_alpha) > 0.0f) {
+        const float ap = aperture_weight(ex, px, pz, a.f_number, a.rx_window, a.tukey_alpha);
+        if (ap > 0.0f) {
           mask |= 1u << k;
           r = dist3(ex, 0.0f, 0.0f, px, py, pz) / a.c;
+          // The weight waits in the channel's slot of the pass's values.
+          if (kSum) ys[(cq * kG + k) * kPx + pl].x = ap;
         }
       }
       if (k & 1)
@@ -691,7 +697,7 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
         const int ch = g + k;
         float2 y = make_float2(0.f, 0.f);
         if ((mask >> k) & 1u) {
-          const float ap = aperture_weight(elem_x(a, ch), px, pz, a.f_number, a.rx_window, a.tukey_alpha);
+          const float ap = ys[(cq * kG + k) * kPx + pl].x;
           float rc = 1.0f, rs = 0.0f;
           if (a.fdem > 0.0f) sincosf(a.two_pi_f * ((k & 1) ? rt[k / 2].y : rt[k / 2].x), &rs, &rc);
           const float gr = ap * rc, gi = ap * rs;
