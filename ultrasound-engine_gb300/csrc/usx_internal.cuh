@@ -342,8 +342,6 @@ int lmv_subspace_record_bytes(int n_beams);
 bool gemm_tc5_supported(int M, int N, int K);
 int launch_gemm_tc5(usx_ctx* ctx, const void* A, const void* Bt, const float* bias, bool relu, void* C16, float* C32,
                     int M, int N, int K);
-// wt[N][K] = w[K][N] (BF16).
-int transpose_bf16(cudaStream_t st, const void* w, int K, int N, void* wt);
 
 // The network (mlp.cu). mlp_infer runs `rows` (a multiple of 128) BF16 input
 // rows through every layer with caller scratch t0, t1 (rows x widest BF16
