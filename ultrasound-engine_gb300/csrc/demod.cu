@@ -1,27 +1,36 @@
 // demod.cu — quadrature demodulation + decimating FIR (reference
-// demodulate.cpp:36-121), HBM-bound.
+// demodulate.cpp:36-121).
 //
 // Layout: RF [trace][n_in] float -> IQ [trace][n_out] complex, trace =
 // event*n_channels + channel.
 //
-// demod_slide_kernel<NT> (no decimation, NT taps; the default 33-tap filter):
-// a block of 8 warps owns 8 traces x 256 output samples. It stages the 288
-// input samples those outputs need for each trace in shared memory, already
-// mixed to baseband (the rotator once per block for all 8 traces), with one
-// pad word every 8 samples so that lanes reading 8-sample strides hit distinct
-// banks. Each warp then filters one trace: lane l produces outputs 8l..8l+7
-// from one descending pass over its 8+NT-1 window samples, each sample read
-// from shared memory once and multiplied into every output it reaches (the
-// taps are compile-time constant-bank operands). Every output still sums its
+// demod_slide_kernel<NT, R> (no decimation, NT taps; the default 33-tap filter):
+// a warp filters a segment of 32 R output samples of up to four traces in
+// turn; the block's eight warps share the segment's rotator. The 32 R + NT - 1
+// input samples go to the warp's own row of shared memory already mixed to
+// baseband (a lane's samples are lane + 32 m: no index arithmetic, and the next
+// trace's are fetched behind the filter). Lane l then produces outputs R l ..
+// R l + R - 1 from one descending pass over its R + NT - 1 window samples, each
+// sample read from shared memory once and multiplied into every output it
+// reaches (the taps are compile-time constant-bank operands); R is odd, so that
+// lanes reading R-sample strides hit distinct banks. Every output still sums its
 // taps in ascending order, as the reference does. The outputs go back through
 // the warp's own shared-memory row so the IQ stores are coalesced. Samples
 // outside the trace are staged as zeros: an output whose tap range the
 // reference clips (j_lo > 0 or j_hi < NT-1) then adds exact zeros outside
 // that range, which leaves its sum unchanged.
+// 75 x 128 traces x 2,073 samples: 55 us (239 MB at 4.3 TB/s), where staging by
+// the whole block with a division per sample and eight outputs per lane took 82;
+// bound by issue (the 33 packed FMAs per output alone are 35 us of FP32 pipe).
+// Three blocks per SM 57.8 us, five (51 registers) 63.7, taps stored twice as
+// packed operands the same.
 //
 // demod_kernel (any decimation or tap count): a block owns 8 traces x 128
 // outputs, one output per thread per trace, taps read from the parameter
-// block in a runtime loop.
+// block in a runtime loop, the eight traces' sums side by side in it (one
+// trace after the other was a single chain of dependent FMAs): 75 x 128 traces
+// x 2,073 samples, 47 taps 304 -> 213 us; 33 taps, decimation 4 255 -> 154 us.
+// Bound by shared memory, one 8-byte read per tap.
 //
 // Arithmetic follows the reference term by term (mix, then tap product and
 // accumulation in ascending tap order, then x2); the tap product and the
@@ -47,6 +56,7 @@ struct DemodParams {
   int n_in, n_out, dec, n_taps, gd;
   float neg_two_pi_f;   // -2*pi*fdem, float-rounded as the reference folds it
   float t0, fs;
+  int per_warp;         // traces a warp filters in turn (demod_slide_kernel)
   float h[kMaxTaps];
 };
 
@@ -73,15 +83,16 @@ __global__ void __launch_bounds__(kOut) demod_kernel(const DemodParams p) {
     }
     rot[s] = r;
   }
-  __syncthreads();
-  for (int q = threadIdx.x; q < kTraces * span; q += blockDim.x) {
-    const int t = q / span, s = q - t * span;
-    const long tr = tr0 + t;
+  for (int s = threadIdx.x; s < span; s += kOut) {
     const int n = n_base + s;
-    float x = 0.f;
-    if (tr < p.n_traces && n >= 0 && n < p.n_in) x = __ldg(p.rf + tr * p.n_in + n);
-    const float2 r = rot[s];
-    mixed[q] = make_float2(r.x * x, r.y * x);
+    const bool in = n >= 0 && n < p.n_in;
+    const float2 r = rot[s];   // this thread's own
+    float x[kTraces];
+#pragma unroll
+    for (int t = 0; t < kTraces; ++t)
+      x[t] = in && tr0 + t < p.n_traces ? __ldg(p.rf + (tr0 + t) * p.n_in + n) : 0.f;
+#pragma unroll
+    for (int t = 0; t < kTraces; ++t) mixed[t * span + s] = make_float2(r.x * x[t], r.y * x[t]);
   }
   __syncthreads();
 
@@ -91,42 +102,51 @@ __global__ void __launch_bounds__(kOut) demod_kernel(const DemodParams p) {
   const int j_lo = max(0, centre - p.n_in + 1);
   const int j_hi = min(p.n_taps - 1, centre);
   // mixed index of input sample (centre - j) is centre - j - n_base.
-  const int off = centre - n_base;
+  const float2* m = mixed + (centre - n_base);
+  float2 acc[kTraces];
 #pragma unroll
-  for (int t = 0; t < kTraces; ++t) {
-    const long tr = tr0 + t;
-    if (tr >= p.n_traces) break;
-    const float2* m = mixed + t * span;
-    float ar = 0.f, ai = 0.f;
-    for (int j = j_lo; j <= j_hi; ++j) {
-      const float2 v = m[off - j];
-      const float hj = p.h[j];
-      ar = fmaf(v.x, hj, ar);
-      ai = fmaf(v.y, hj, ai);
-    }
-    p.iq[tr * p.n_out + k] = make_float2(ar * 2.0f, ai * 2.0f);
+  for (int t = 0; t < kTraces; ++t) acc[t] = make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (int j = j_lo; j <= j_hi; ++j) {
+    const float2 h = make_float2(p.h[j], p.h[j]);
+#pragma unroll
+    for (int t = 0; t < kTraces; ++t) acc[t] = __ffma2_rn(m[t * span - j], h, acc[t]);
   }
+#pragma unroll
+  for (int t = 0; t < kTraces; ++t)
+    if (tr0 + t < p.n_traces) p.iq[(tr0 + t) * p.n_out + k] = make_float2(acc[t].x * 2.0f, acc[t].y * 2.0f);
 }
 
-constexpr int kSlideR = 8;                       // outputs per lane
-constexpr int kSlideWarps = 8;                   // traces per block
-constexpr int kSlideOut = 32 * kSlideR;          // outputs per trace segment
+constexpr int kSlideWarps = 8;                   // traces of a block in flight
 
-// Shared-memory slot of window sample s: one pad word after every 8 samples.
-__device__ __forceinline__ int slide_pos(int s) { return s + (s >> 3); }
+template <int NT, int R>
+__global__ void __launch_bounds__(32 * kSlideWarps, 4) demod_slide_kernel(const __grid_constant__ DemodParams p) {
+  constexpr int W = 32 * R + NT - 1;             // window samples per trace
+  constexpr int kPer = (W + 31) / 32;
+  __shared__ float2 rot[kPer * 32];
+  __shared__ float2 mixed[kSlideWarps][kPer * 32];
 
-template <int NT>
-__global__ void __launch_bounds__(32 * kSlideWarps) demod_slide_kernel(const DemodParams p) {
-  constexpr int W = kSlideOut + NT - 1;          // window samples per trace
-  constexpr int ROW = W + W / 8 + 1;             // padded row length (float2)
-  __shared__ float2 rot[W];
-  __shared__ float2 mixed[kSlideWarps][ROW];
-
-  const int k0 = blockIdx.y * kSlideOut;
-  const long tr0 = static_cast<long>(blockIdx.x) * kSlideWarps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k0 = blockIdx.y * 32 * R;
   const int n_base = k0 + p.gd - (NT - 1);       // input index of window sample 0
+  const long tr_end = min(p.n_traces, (blockIdx.x + 1L) * kSlideWarps * p.per_warp);
+  long tr = blockIdx.x * static_cast<long>(kSlideWarps) * p.per_warp + warp;
 
-  for (int s = threadIdx.x; s < W; s += blockDim.x) {
+  // A lane's samples are lane + 32 m of every trace.
+  unsigned in = 0;
+#pragma unroll
+  for (int m = 0; m < kPer; ++m) {
+    const int n = n_base + lane + 32 * m;
+    if (n >= 0 && n < p.n_in) in |= 1u << m;
+  }
+  float x[kPer];
+  auto fetch = [&](long t) {
+    const float* src = p.rf + t * p.n_in + n_base + lane;
+#pragma unroll
+    for (int m = 0; m < kPer; ++m) x[m] = (in >> m & 1u) ? __ldg(src + 32 * m) : 0.f;
+  };
+  if (tr < tr_end) fetch(tr);
+  for (int s = threadIdx.x; s < kPer * 32; s += 32 * kSlideWarps) {
     const int n = n_base + s;
     float2 r = make_float2(0.f, 0.f);
     if (n >= 0 && n < p.n_in) {
@@ -138,61 +158,78 @@ __global__ void __launch_bounds__(32 * kSlideWarps) demod_slide_kernel(const Dem
     }
     rot[s] = r;
   }
-  // Raw samples first (independent loads in flight), then mix once the rotator is in.
-  constexpr int kPer = (kSlideWarps * W + 32 * kSlideWarps - 1) / (32 * kSlideWarps);
-  float x[kPer];
-#pragma unroll
-  for (int m = 0; m < kPer; ++m) {
-    const int q = threadIdx.x + m * 32 * kSlideWarps;
-    const int t = q / W, s = q - t * W;
-    const long tr = tr0 + t;
-    const int n = n_base + s;
-    x[m] = (q < kSlideWarps * W && tr < p.n_traces && n >= 0 && n < p.n_in) ? __ldg(p.rf + tr * p.n_in + n) : 0.f;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int m = 0; m < kPer; ++m) {
-    const int q = threadIdx.x + m * 32 * kSlideWarps;
-    if (q < kSlideWarps * W) {
-      const int t = q / W, s = q - t * W;
-      const float2 r = rot[s];
-      mixed[t][slide_pos(s)] = make_float2(r.x * x[m], r.y * x[m]);
-    }
-  }
   __syncthreads();
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long tr = tr0 + warp;
-  if (tr >= p.n_traces) return;
   float2* row = mixed[warp];
-  // (re, im) of each output accumulate as one packed pair (two FP32 FMAs per
-  // instruction, each rounded as fmaf).
-  float2 acc[kSlideR];
+  for (; tr < tr_end; tr += kSlideWarps) {
 #pragma unroll
-  for (int r = 0; r < kSlideR; ++r) acc[r] = make_float2(0.f, 0.f);
-  // Window sample i of this lane is s = 8*lane + i; output r uses tap
-  // j = r + NT - 1 - i, so descending i visits each output's taps in ascending j.
-#pragma unroll
-  for (int i = kSlideR + NT - 2; i >= 0; --i) {
-    const float2 v = row[slide_pos(kSlideR * lane + i)];
-#pragma unroll
-    for (int r = 0; r < kSlideR; ++r) {
-      const int j = r + NT - 1 - i;
-      if (j >= 0 && j < NT) acc[r] = __ffma2_rn(v, make_float2(p.h[j], p.h[j]), acc[r]);
+    for (int m = 0; m < kPer; ++m) {
+      const float2 r = rot[lane + 32 * m];
+      row[lane + 32 * m] = make_float2(r.x * x[m], r.y * x[m]);
     }
-  }
-  __syncwarp();
+    __syncwarp();
+    if (tr + kSlideWarps < tr_end) fetch(tr + kSlideWarps);   // the next trace's, behind the filter
+    // (re, im) of each output accumulate as one packed pair (two FP32 FMAs per
+    // instruction, each rounded as fmaf).
+    float2 acc[R];
 #pragma unroll
-  for (int r = 0; r < kSlideR; ++r)
-    row[slide_pos(kSlideR * lane + r)] = make_float2(acc[r].x * 2.0f, acc[r].y * 2.0f);
-  __syncwarp();
-  float2* dst = p.iq + tr * p.n_out + k0;
-  const int n_here = min(kSlideOut, p.n_out - k0);
+    for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+    // Window sample i of this lane is s = R * lane + i; output r uses tap
+    // j = r + NT - 1 - i, so descending i visits each output's taps in ascending j.
 #pragma unroll
-  for (int q = 0; q < kSlideR; ++q) {
-    const int o = lane + 32 * q;
-    if (o < n_here) dst[o] = row[slide_pos(o)];
+    for (int i = R + NT - 2; i >= 0; --i) {
+      const float2 v = row[R * lane + i];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int j = r + NT - 1 - i;
+        if (j >= 0 && j < NT) acc[r] = __ffma2_rn(v, make_float2(p.h[j], p.h[j]), acc[r]);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) row[R * lane + r] = make_float2(acc[r].x * 2.0f, acc[r].y * 2.0f);
+    __syncwarp();
+    float2* dst = p.iq + tr * p.n_out + k0 + lane;
+    const int n_here = p.n_out - k0 - lane;
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+      if (32 * q < n_here) dst[32 * q] = row[lane + 32 * q];
+    __syncwarp();
   }
+}
+
+template <int NT, int R>
+int launch_slide(usx_ctx* ctx, DemodParams& p) {
+  const int gy = ceil_div(p.n_out, 32 * R);
+  // Up to four traces per warp while eight blocks per SM (two waves) remain.
+  p.per_warp = static_cast<int>(std::max(1L, std::min(4L, p.n_traces * gy / (kSlideWarps * 8L * ctx->sm_count))));
+  const long per_block = static_cast<long>(kSlideWarps) * p.per_warp;
+  const long gx = (p.n_traces + per_block - 1) / per_block;
+  if (gx > 0x7fffffffL || gy > 65535) return fail(USX_ERR_UNSUPPORTED, "usx_cu_demodulate: acquisition too large");
+  prof_begin(ctx, "demod_slide_kernel");
+  demod_slide_kernel<NT, R>
+      <<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), 32 * kSlideWarps, 0, ctx->stream>>>(p);
+  prof_end(ctx);
+  USX_CHECK_LAUNCH("demod_slide_kernel");
+  return USX_OK;
+}
+
+// Outputs per lane: the time follows the outputs with their padding (segments x
+// R), so the R with the fewest; the larger on a tie, which reads less of the
+// window twice. 75 x 128 traces, 33 taps, R = 7 / 9 / 11 / 13: 2,073 samples
+// (70 / 72 / 66 / 65 x 32 outputs) 60.1 / 63.4 / 57.6 / 55.6 us; 1,034 samples
+// (35 / 36 / 33 / 39) 33.5 / 34.9 / 32.9 / 37.0. While the blocks of R = 7 are not
+// four per SM a warp's own chain counts, and the shortest is R = 7 (32 traces
+// of 660 samples 4.3 us, with R = 11 6.1).
+template <int NT>
+int launch_slide_r(usx_ctx* ctx, DemodParams& p) {
+  auto cost = [&](int r) { return ceil_div(p.n_out, 32 * r) * r; };
+  const long blocks = (p.n_traces + kSlideWarps - 1) / kSlideWarps * ceil_div(p.n_out, 32 * 7);
+  if (blocks > 4L * ctx->sm_count) {
+    if (cost(13) <= cost(11) && cost(13) <= cost(7)) return launch_slide<NT, 13>(ctx, p);
+    if (cost(11) <= cost(7)) return launch_slide<NT, 11>(ctx, p);
+  }
+  return launch_slide<NT, 7>(ctx, p);
 }
 
 }  // namespace
@@ -229,18 +266,7 @@ extern "C" int usx_cu_demodulate(usx_ctx* ctx, const usx_channel_desc* cd,
   p.fs = fs;
   if (out_fdem) *out_fdem = fdem;
   if (dec == 1 && (n_taps == 33 || n_taps == 21)) {
-    const long gx = (p.n_traces + kSlideWarps - 1) / kSlideWarps;
-    const int gy = ceil_div(p.n_out, kSlideOut);
-    if (gx > 0x7fffffffL || gy > 65535) return fail(USX_ERR_UNSUPPORTED, "usx_cu_demodulate: acquisition too large");
-    dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    prof_begin(ctx, "demod_slide_kernel");
-    if (n_taps == 33)
-      demod_slide_kernel<33><<<grid, 32 * kSlideWarps, 0, ctx->stream>>>(p);
-    else
-      demod_slide_kernel<21><<<grid, 32 * kSlideWarps, 0, ctx->stream>>>(p);
-    prof_end(ctx);
-    USX_CHECK_LAUNCH("demod_slide_kernel");
-    return USX_OK;
+    return n_taps == 33 ? launch_slide_r<33>(ctx, p) : launch_slide_r<21>(ctx, p);
   }
   const int span = kOut * dec + n_taps - 1;
   const size_t smem = sizeof(float2) * static_cast<size_t>(span) * (1 + kTraces);

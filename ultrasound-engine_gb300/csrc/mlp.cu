@@ -4,7 +4,7 @@
 // GEMMs and Adam.
 //
 // GEMM: C[M x N] (+)= op(A)[M x K] * op(B)[K x N], BF16 operands, FP32
-// accumulators, mma.sync m16n8k16 fed by ldmatrix from a two-stage cp.async
+// accumulators, mma.sync m16n8k16 fed by ldmatrix from a four-stage cp.async
 // shared-memory pipeline. 128 x 128 x 32 block tiles, 8 warps of 64 x 32.
 // Operand layouts cover the three products of training:
 //   forward   H = X W        A row-major (k contiguous), B row-major (n contiguous)
