@@ -1209,10 +1209,14 @@ __global__ void __launch_bounds__(32 * kWarpMvWarps) mv_warp_kernel(const MvWarp
 // Factorisation: panels of four or eight columns. A lane holds the panel entries
 // of rows c0 + lane + 32 s in registers (pivots and multipliers by shuffles),
 // leaves the panel in shared memory, and updates its own rows of the trailing
-// triangle by that rank in FP32 pairs.
+// triangle by that rank in FP32 pairs. A panel runs over as many row slots as its
+// remaining rows fill (all of the first panel's 7.98 ms; with the doubled operand
+// on the lane's own side, no moves per column, 7.91; the multipliers' shuffles off
+// the chain of pivots 7.77; registers for 14 CTAs at four columns 7.65).
 //
-// 128 channels, 75 plane waves, 512 x 1024 pixels, L up to 64: 8.0 ms against
-// 15.5 for mv_warp_kernel (staging 2.3, covariance with both products of every
+// 128 channels, 75 plane waves, 512 x 1024 pixels, L up to 64: 7.65 ms (staging
+// 1.2, covariance 2.7, panels 1.5, trailing rows 2.3) against 15.5 for
+// mv_warp_kernel (staging 2.3, covariance with both products of every
 // step 3.4, factor with its panels in shared memory 5.7, substitutions 4.1). What
 // bounds it: the shared-memory pipe for L of 17 to 48 (the trailing rows' reads
 // and writes; 75% of its wavefronts with panels of four), latency at 10 warps
@@ -1249,109 +1253,128 @@ __device__ __forceinline__ float2 shfl2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
+// One panel of chol_augmented, columns c0 .. c0 + kW - 1, whose rows c0 .. L + 1
+// fit kS slots of a lane.
+template <int kS, int kW>
+__device__ __forceinline__ bool chol_panel(float2* Rl, float2* Rx, int lx, float4* P, int L, int lane, int c0) {
+  const int nb = min(kW, L - c0);
+  float2 v[kS][kW];
+  float2* row[kS];
+#pragma unroll
+  for (int s = 0; s < kS; ++s) {
+    const int i = c0 + lane + 32 * s;
+    row[s] = i < L ? Rl + tri(i, 0) : Rx + (i == L ? 0 : lx);
+#pragma unroll
+    for (int c = 0; c < kW; ++c)
+      v[s][c] = c < nb && i < L + 2 && (s > 0 || lane >= c) ? row[s][c0 + c] : make_float2(0.f, 0.f);
+  }
+#pragma unroll
+  for (int c = 0; c < kW; ++c) {
+    if (c >= nb) break;
+    // The multipliers are read before the pivot's root is known: v / d times the
+    // unscaled conj(v_cc) keeps their shuffles off the chain of pivots.
+    const float d = __shfl_sync(0xffffffffu, v[0][c].x, c);
+    float2 m[kW];
+#pragma unroll
+    for (int cc = c + 1; cc < kW; ++cc) m[cc] = shfl2(v[0][c], cc);
+    if (!(d > 0.0f)) return false;
+    float inv = rsqrtf(d);
+    inv = inv * fmaf(-0.5f * d * inv, inv, 1.5f);
+#pragma unroll
+    for (int s = 0; s < kS; ++s) {
+      v[s][c] = make_float2(v[s][c].x * inv, v[s][c].y * inv);
+      const float2 u = make_float2(v[s][c].x * inv, v[s][c].y * inv);
+#pragma unroll
+      for (int cc = c + 1; cc < kW; ++cc) {
+        if (cc >= nb) break;
+        v[s][cc].x = fmaf(-u.x, m[cc].x, fmaf(-u.y, m[cc].y, v[s][cc].x));
+        v[s][cc].y = fmaf(-u.y, m[cc].x, fmaf(u.x, m[cc].y, v[s][cc].y));
+      }
+    }
+  }
+  const int k0 = c0 + nb;
+#pragma unroll
+  for (int s = 0; s < kS; ++s) {
+    const int i = c0 + lane + 32 * s;
+    if (i < k0 || i >= L + 2) continue;
+    if (i < L) {
+#pragma unroll
+      for (int c = 0; c < kW; c += 2)
+        P[kW / 2 * i + c / 2] = make_float4(-v[s][c].x, -v[s][c].y, -v[s][c + 1].x, -v[s][c + 1].y);
+    } else {
+#pragma unroll
+      for (int c = 0; c < kW; ++c)
+        if (c < nb) row[s][c0 + c] = v[s][c];
+    }
+  }
+  __syncwarp();
+  if (k0 >= L) return true;
+  // Trailing rows: R[i][k] -= sum_c v_ic conj(v_kc), k0 <= k <= min(i, L - 1). The
+  // lane's own v_ic are the pairs' doubled operand, made once per panel: with
+  // A = sum (re v, re v) p and B = sum (im v, im v) p of the (negated) panel
+  // entries p = v_kc as they are read, v conj(p) = (A.x + B.y, B.x - A.y).
+  float2 vr[kS][kW], vi[kS][kW];
+  int last[kS];
+#pragma unroll
+  for (int s = 0; s < kS; ++s) {
+    const int i = c0 + lane + 32 * s;
+    last[s] = i >= k0 && i < L + 2 ? min(i, L - 1) : -1;
+#pragma unroll
+    for (int c = 0; c < kW; ++c) {
+      vr[s][c] = make_float2(v[s][c].x, v[s][c].x);
+      vi[s][c] = make_float2(v[s][c].y, v[s][c].y);
+    }
+  }
+  auto update = [&](auto from, int k_lo, int k_hi) {
+    constexpr int S0 = decltype(from)::value;   // the slots below are done
+#pragma unroll 2
+    for (int k = k_lo; k <= k_hi; ++k) {
+      float2 pk[kW];
+#pragma unroll
+      for (int c = 0; c < kW; c += 2) {
+        const float4 p = P[kW / 2 * k + c / 2];
+        pk[c] = make_float2(p.x, p.y);
+        pk[c + 1] = make_float2(p.z, p.w);
+      }
+#pragma unroll
+      for (int s = S0; s < kS; ++s) {
+        if (k > last[s]) continue;
+        const float2 r = row[s][k];
+        float2 A = __fmul2_rn(vr[s][0], pk[0]), B = __fmul2_rn(vi[s][0], pk[0]);
+#pragma unroll
+        for (int c = 1; c < kW; ++c) {
+          A = __ffma2_rn(vr[s][c], pk[c], A);
+          B = __ffma2_rn(vi[s][c], pk[c], B);
+        }
+        row[s][k] = make_float2(r.x + (A.x + B.y), r.y + (B.x - A.y));
+      }
+    }
+  };
+  update(std::integral_constant<int, 0>{}, k0, min(L - 1, c0 + 31));
+  if constexpr (kS > 1) update(std::integral_constant<int, 1>{}, max(k0, c0 + 32), L - 1);
+  __syncwarp();
+  return true;
+}
+
 // Factors the packed lower triangle Rl (L rows) with the two right-hand rows
 // Rx[0..L) and Rx[lx..lx + L), which become y^H and z^H (see above). P: the panel,
 // negated, kW complex per row. False on a non-positive pivot.
 template <int kPan, int kW>
 __device__ __forceinline__ bool chol_augmented(float2* Rl, float2* Rx, int lx, float4* P, int L, int lane) {
-  for (int c0 = 0; c0 < L; c0 += kW) {
-    const int nb = min(kW, L - c0);
-    float2 v[kPan][kW];
-    float2* row[kPan];
-#pragma unroll
-    for (int s = 0; s < kPan; ++s) {
-      const int i = c0 + lane + 32 * s;
-      row[s] = i < L ? Rl + tri(i, 0) : Rx + (i == L ? 0 : lx);
-#pragma unroll
-      for (int c = 0; c < kW; ++c)
-        v[s][c] = c < nb && i < L + 2 && (s > 0 || lane >= c) ? row[s][c0 + c] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int c = 0; c < kW; ++c) {
-      if (c >= nb) break;
-      const float d = __shfl_sync(0xffffffffu, v[0][c].x, c);
-      if (!(d > 0.0f)) return false;
-      float inv = rsqrtf(d);
-      inv = inv * fmaf(-0.5f * d * inv, inv, 1.5f);
-#pragma unroll
-      for (int s = 0; s < kPan; ++s) v[s][c] = make_float2(v[s][c].x * inv, v[s][c].y * inv);
-#pragma unroll
-      for (int cc = c + 1; cc < kW; ++cc) {
-        if (cc >= nb) break;
-        const float2 m = shfl2(v[0][c], cc);
-#pragma unroll
-        for (int s = 0; s < kPan; ++s) {
-          v[s][cc].x = fmaf(-v[s][c].x, m.x, fmaf(-v[s][c].y, m.y, v[s][cc].x));
-          v[s][cc].y = fmaf(-v[s][c].y, m.x, fmaf(v[s][c].x, m.y, v[s][cc].y));
-        }
-      }
-    }
-    const int k0 = c0 + nb;
-#pragma unroll
-    for (int s = 0; s < kPan; ++s) {
-      const int i = c0 + lane + 32 * s;
-      if (i < k0 || i >= L + 2) continue;
-      if (i < L) {
-#pragma unroll
-        for (int c = 0; c < kW; c += 2)
-          P[kW / 2 * i + c / 2] = make_float4(-v[s][c].x, -v[s][c].y, -v[s][c + 1].x, -v[s][c + 1].y);
-      } else {
-#pragma unroll
-        for (int c = 0; c < kW; ++c)
-          if (c < nb) row[s][c0 + c] = v[s][c];
-      }
-    }
-    __syncwarp();
-    if (k0 >= L) break;
-    // Trailing rows: R[i][k] -= sum_c v_ic conj(v_kc), k0 <= k <= min(i, L - 1).
-    float2 f2[kPan][kW];   // v times -j
-    int last[kPan];
-#pragma unroll
-    for (int s = 0; s < kPan; ++s) {
-      const int i = c0 + lane + 32 * s;
-      last[s] = i >= k0 && i < L + 2 ? min(i, L - 1) : -1;
-#pragma unroll
-      for (int c = 0; c < kW; ++c) {
-        f2[s][c] = make_float2(v[s][c].y, -v[s][c].x);
-      }
-    }
-    auto update = [&](auto from, int k_lo, int k_hi) {
-      constexpr int S0 = decltype(from)::value;   // the slots below are done
-#pragma unroll 2
-      for (int k = k_lo; k <= k_hi; ++k) {
-        // (The pairs are made here: stored as (re, re, im, im) the reads cost
-        // more than the moves, 11.9 against 11.2 ms per frame.)
-        float2 p1[kW], p2[kW];
-#pragma unroll
-        for (int c = 0; c < kW; c += 2) {
-          const float4 p = P[kW / 2 * k + c / 2];
-          p1[c] = make_float2(p.x, p.x);
-          p2[c] = make_float2(p.y, p.y);
-          p1[c + 1] = make_float2(p.z, p.z);
-          p2[c + 1] = make_float2(p.w, p.w);
-        }
-#pragma unroll
-        for (int s = S0; s < kPan; ++s) {
-          if (k > last[s]) continue;
-          float2 r = row[s][k];
-#pragma unroll
-          for (int c = 0; c < kW; ++c) {
-            r = __ffma2_rn(v[s][c], p1[c], r);
-            r = __ffma2_rn(f2[s][c], p2[c], r);
-          }
-          row[s][k] = r;
-        }
-      }
-    };
-    update(std::integral_constant<int, 0>{}, k0, min(L - 1, c0 + 31));
-    if constexpr (kPan > 1) update(std::integral_constant<int, 1>{}, max(k0, c0 + 32), L - 1);
-    __syncwarp();
-  }
+  int c0 = 0;
+  if constexpr (kPan > 2)
+    for (; c0 < L && L + 2 - c0 > 64; c0 += kW)
+      if (!chol_panel<3, kW>(Rl, Rx, lx, P, L, lane, c0)) return false;
+  if constexpr (kPan > 1)
+    for (; c0 < L && L + 2 - c0 > 32; c0 += kW)
+      if (!chol_panel<2, kW>(Rl, Rx, lx, P, L, lane, c0)) return false;
+  for (; c0 < L; c0 += kW)
+    if (!chol_panel<1, kW>(Rl, Rx, lx, P, L, lane, c0)) return false;
   return true;
 }
 
 template <int kPan, int kW>
-__global__ void __launch_bounds__(32 * kMvFp32Warps) mv_fp32_kernel(const MvWarpArgs wa) {
+__global__ void __launch_bounds__(32 * kMvFp32Warps, kW == 4 ? 14 : 1) mv_fp32_kernel(const MvWarpArgs wa) {
   extern __shared__ float4 mvw_smem_raw[];
   const MvTcArgs& a = wa.base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
