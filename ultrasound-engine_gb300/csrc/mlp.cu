@@ -239,6 +239,27 @@ __global__ void f32_to_bf16_kernel(const float* x, __nv_bfloat16* y, long n) {
   if (i < n) y[i] = __float2bfloat16_rn(x[i]);
 }
 
+// A training step's start in one launch: the batch to BF16 (four values per
+// thread), the gradient and the loss to zero.
+__global__ void __launch_bounds__(256) begin_step_kernel(const float* x, __nv_bfloat16* y, long n, float* grad,
+                                                         long n_grad, float* loss) {
+  const long i = 4 * (blockIdx.x * 256L + threadIdx.x);
+  if (i < n) {   // n is a multiple of 128 x 128, and y a whole allocation
+    float v[4];
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+      const float4 q = *reinterpret_cast<const float4*>(x + i);
+      v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = x[i + k];
+    }
+    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+    *reinterpret_cast<uint2*>(y + i) = *reinterpret_cast<const uint2*>(h);
+  }
+  if (i < n_grad) *reinterpret_cast<float4*>(grad + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i == 0) *loss = 0.f;
+}
+
 // Deterministic uniform(-a, a) initialisation from a counter hash.
 __global__ void init_uniform_kernel(float* p, long n, float a, unsigned long long seed) {
   const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
@@ -252,36 +273,27 @@ __global__ void init_uniform_kernel(float* p, long n, float a, unsigned long lon
 }
 
 // dY = 2 (Y - T) * mask / count over the valid outputs; loss sum into *loss.
-// Bound by latency: one loss atomic per block over a bounded grid (5.7 us at
-// 4,096 x 128; an atomic per warp onto the one word, 16,384 of them, 26.7 us).
-// The loss is within 6e-7 of the 64-bit sum of the same outputs (512 to 8,192
-// rows; with an atomic per warp within 3.4e-6).
-constexpr int kMseThreads = 256, kMseBlocks = 512;
-__global__ void __launch_bounds__(kMseThreads)
-    mse_grad_kernel(const float* y, const float* t, const float* mask, long rows, int n_out, int ld, float inv_count,
-                    float* dy32, __nv_bfloat16* dy16, float* loss) {
-  __shared__ float warp_sum[8];
+// Bound by the loss's atomics, one per warp onto one word (26.7 us at 4,096 x 128).
+// Block sums take 5.7 us, but round the total another way: 5 of 60 batches then
+// lie 1.5 times further from the 64-bit loss (its BF16 error of 1e-6 to 2e-5
+// included), 1 of 60 from one run of this kernel to the next.
+__global__ void mse_grad_kernel(const float* y, const float* t, const float* mask, long rows, int n_out,
+                                int ld, float inv_count, float* dy32, __nv_bfloat16* dy16, float* loss) {
+  const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
   float l = 0.f;
-  for (long i = blockIdx.x * static_cast<long>(kMseThreads) + threadIdx.x; i < rows * n_out;
-       i += static_cast<long>(gridDim.x) * kMseThreads) {
+  if (i < rows * n_out) {
     const long r = i / n_out;
     const int c = static_cast<int>(i - r * n_out);
     const long off = r * ld + c;
     const float m = mask ? mask[off] : 1.0f;
     const float d = (y[off] - t[off]) * m;
-    l += d * d * inv_count;
+    l = d * d;
     const float gr = 2.0f * d * inv_count;
     if (dy32) dy32[off] = gr;
     dy16[off] = __float2bfloat16_rn(gr);
   }
   for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = l;
-  __syncthreads();
-  if (threadIdx.x == 0 && loss) {
-    float s = 0.f;
-    for (int w = 0; w < kMseThreads / 32; ++w) s += warp_sum[w];
-    atomicAdd(loss, s);
-  }
+  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, l * inv_count);
 }
 
 // Learned-MV output loss, one warp per row. The network's 128 outputs are 64
@@ -935,11 +947,10 @@ int usx_cu_mlp_train_step(usx_mlp* n, const float* x, const float* target, const
   cudaStream_t st = n->ctx->stream;
   const int L = n->n_layers;
   const long nin = static_cast<long>(rows) * n->dims[0];
-  f32_to_bf16_kernel<<<ceil_div(nin, 256), 256, 0, st>>>(x, n->act[0], nin);
-  USX_CHECK_LAUNCH("f32_to_bf16_kernel");
+  const long n_grad = static_cast<long>(n->n_params);   // a multiple of 128
+  begin_step_kernel<<<ceil_div(std::max(nin, n_grad), 1024), 256, 0, st>>>(x, n->act[0], nin, n->grad, n_grad, n->loss);
+  USX_CHECK_LAUNCH("begin_step_kernel");
   if (int rc = mlp_forward_rows(n, rows)) return rc;
-  USX_CUDA(cudaMemsetAsync(n->grad, 0, sizeof(float) * n->n_params, st));
-  USX_CUDA(cudaMemsetAsync(n->loss, 0, sizeof(float), st));
   const int n_out = n->dims.back();
   if (n->loss_kind == USX_MLP_LOSS_LMV_SUBSPACE) {
     lmv_subspace_loss_kernel<<<ceil_div(static_cast<long>(rows) * 32, 256), 256, 0, st>>>(
@@ -952,8 +963,7 @@ int usx_cu_mlp_train_step(usx_mlp* n, const float* x, const float* target, const
   } else {
     // Count of valid outputs (mask sum) is taken as rows * n_out when no mask.
     const float inv_count = 1.0f / static_cast<float>(rows * n_out);
-    const int blocks = std::min(kMseBlocks, ceil_div(static_cast<long>(rows) * n_out, kMseThreads));
-    mse_grad_kernel<<<blocks, kMseThreads, 0, st>>>(
+    mse_grad_kernel<<<ceil_div(static_cast<long>(rows) * n_out, 256), 256, 0, st>>>(
         n->out32, target, mask, rows, n_out, n_out, inv_count, nullptr, n->g16a, n->loss);
     USX_CHECK_LAUNCH("mse_grad_kernel");
   }
