@@ -1,7 +1,7 @@
 """The network's kernels at the sizes where their splits change: the forward
 GEMM's columns over CTAs (few row tiles), the backward launch's three parts
-(input gradient, weight gradient split along the rows, bias sums), the loss
-over a bounded grid, and the transposed weights of a network with more layers
+(input gradient, weight gradient split along the rows, bias sums), the loss,
+and the transposed weights of a network with more layers
 than one launch takes. Oracle: oracle/mlp_oracle.py (same BF16 roundings,
 float64 sums)."""
 
