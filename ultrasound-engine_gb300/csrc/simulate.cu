@@ -280,7 +280,11 @@ __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs 
         centre = (t_arr - inc_t0) * a.fs_os;
       }
       const float whole = floorf(centre), frac = centre - whole;
-      e_tab[q] = make_float4(amp, frac, 1.0f - frac, __int_as_float(static_cast<int>(whole) - a.pulse_n / 2));
+      // A pulse seconds past the window (a delay is the caller's, an infinite
+      // one too) stays far outside it: within +-2^30, so that no slot index
+      // formed from the base wraps back into range.
+      const int slot = max(-(1 << 30), min(1 << 30, static_cast<int>(whole)));
+      e_tab[q] = make_float4(amp, frac, 1.0f - frac, __int_as_float(slot - a.pulse_n / 2));
     }
     __syncwarp();
     for (int q = 0; q < n_act; ++q) {
