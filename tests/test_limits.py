@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from gold import rel_l2
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +50,23 @@ def test_an_element_fired_outside_the_window_adds_nothing(gpu, late):
     want = pulse_echo(capi, torch, ctx, np.zeros_like(delays), apod)
     assert np.isfinite(got).all() and np.abs(want).max() > 0
     assert rel_l2(got, want) < 1e-6
+
+
+@pytest.mark.parametrize("n_smp,taps", [(14679840, 33), (14680064, 33), (14680064, 21)])
+def test_demodulation_of_the_longest_traces(gpu, oracle, n_smp, taps):
+    """65,535 segments of 224 outputs, and one more: against the oracle, tap by
+    tap in the same order (1e-5 of the largest output, as at other sizes)."""
+    torch, capi, ctx = gpu
+    rf = np.random.default_rng(6).standard_normal((1, 1, n_smp)).astype(np.float32)
+    z, w = np.zeros((1, 1), np.float32), np.ones((1, 1), np.float32)
+    ch = capi.Channel(capi.Probe(1, 3e-4, 2.7e-4, 5e-3, 5e6, 0.6), capi.Medium(1540.0, 0.5, 1000.0),
+                      capi.Acquisition(2e7, n_smp, 0.0, 5e3), [dict(type=1, angle=0.0, delays=z[0], apodization=w[0])])
+    cd = O.channel_desc(O.probe(n_elements=1, pitch=3e-4, element_width=2.7e-4, center_frequency=5e6, bandwidth=0.6),
+                        O.medium(), O.acquisition(fs=2e7, n_samples=n_smp, prf=5e3),
+                        O.TxSet(np.full(1, 1, np.int32), np.zeros(1, np.float32), np.zeros((1, 3), np.float32),
+                                np.zeros((1, 3), np.float32), z, w))
+    want = oracle.demodulate(cd, O.demod_config(filter_taps=taps), rf)
+    d = torch.from_numpy(rf).cuda()
+    iq = torch.full(want.shape, float("nan"), dtype=torch.complex64, device="cuda")
+    ctx.demodulate(ch, capi.demod_config(filter_taps=taps), d.data_ptr(), iq.data_ptr())
+    assert np.abs(iq.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()

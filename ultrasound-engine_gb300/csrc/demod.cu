@@ -198,6 +198,8 @@ __global__ void __launch_bounds__(32 * kSlideWarps, 4) demod_slide_kernel(const 
   }
 }
 
+constexpr int kMaxSegments = 65535;   // gridDim.y
+
 template <int NT, int R>
 int launch_slide(usx_ctx* ctx, DemodParams& p) {
   const int gy = ceil_div(p.n_out, 32 * R);
@@ -205,7 +207,8 @@ int launch_slide(usx_ctx* ctx, DemodParams& p) {
   p.per_warp = static_cast<int>(std::max(1L, std::min(4L, p.n_traces * gy / (kSlideWarps * 8L * ctx->sm_count))));
   const long per_block = static_cast<long>(kSlideWarps) * p.per_warp;
   const long gx = (p.n_traces + per_block - 1) / per_block;
-  if (gx > 0x7fffffffL || gy > 65535) return fail(USX_ERR_UNSUPPORTED, "usx_cu_demodulate: acquisition too large");
+  if (gx > 0x7fffffffL || gy > kMaxSegments)
+    return fail(USX_ERR_UNSUPPORTED, "usx_cu_demodulate: acquisition too large");
   prof_begin(ctx, "demod_slide_kernel");
   demod_slide_kernel<NT, R>
       <<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), 32 * kSlideWarps, 0, ctx->stream>>>(p);
@@ -225,6 +228,9 @@ template <int NT>
 int launch_slide_r(usx_ctx* ctx, DemodParams& p) {
   auto cost = [&](int r) { return ceil_div(p.n_out, 32 * r) * r; };
   const long blocks = (p.n_traces + kSlideWarps - 1) / kSlideWarps * ceil_div(p.n_out, 32 * 7);
+  // Segments are the grid's second dimension: past its limit with R = 7 (traces
+  // of 14,679,840 samples), the longest segment.
+  if (ceil_div(p.n_out, 32 * 7) > kMaxSegments) return launch_slide<NT, 13>(ctx, p);
   if (blocks > 4L * ctx->sm_count) {
     if (cost(13) <= cost(11) && cost(13) <= cost(7)) return launch_slide<NT, 13>(ctx, p);
     if (cost(11) <= cost(7)) return launch_slide<NT, 11>(ctx, p);
