@@ -497,9 +497,8 @@ __host__ __device__ constexpr size_t exp_smem_bytes(int events, int pixel_warps,
 // Sample indices take floor(idx) by one directed-rounding addition: 2^23 + idx
 // rounded down is 2^23 + floor(idx) for 0 <= idx < 2^23, its low mantissa bits
 // the integer (no conversion instruction, which run at a fraction of the FP32
-// rate). A negative or infinite index, or one of 2^23 and above, gives at least
-// 2^23: past every trace these kernels take. So does NaN: delays that are no
-// numbers are looked for before the index is formed.
+// rate). A negative, infinite or NaN index, or one of 2^23 and above, gives at
+// least 2^23: past every trace these kernels take.
 constexpr int kMaxFastSamples = 1 << 23;
 
 template <int kG, int kPW, int kCQ, int kWL, int kTL, bool kSum>
@@ -570,14 +569,10 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
   __syncthreads();   // (also: the previous tile's shared memory is no longer read)
   if (cq == 0) {
     int c_lo = a.n_ch, c_hi = -1;
-    if (valid && !(pz <= 0.0f)) {
-      // (The half width as aperture_weight has it; a coordinate that is no
-      // number leaves the whole array, whose windows then decide.)
-      const float half = fmaxf(0.5f * pz / fmaxf(a.f_number, 1e-3f), 1e-9f), top = static_cast<float>(a.n_ch - 1);
-      const float lo = floorf((px - half) / a.pitch + a.half_nm1) - 2.0f;
-      const float hi = ceilf((px + half) / a.pitch + a.half_nm1) + 2.0f;
-      c_lo = lo > 0.0f ? static_cast<int>(fminf(lo, top)) : 0;
-      c_hi = hi < top ? static_cast<int>(fmaxf(hi, 0.0f)) : a.n_ch - 1;
+    if (valid && pz > 0.0f) {
+      const float half = 0.5f * pz / fmaxf(a.f_number, 1e-3f), top = static_cast<float>(a.n_ch - 1);
+      c_lo = static_cast<int>(fminf(fmaxf(floorf((px - half) / a.pitch + a.half_nm1) - 2.0f, 0.0f), top));
+      c_hi = static_cast<int>(fminf(fmaxf(ceilf((px + half) / a.pitch + a.half_nm1) + 2.0f, 0.0f), top));
     }
     c_lo = __reduce_min_sync(0xffffffffu, c_lo);
     c_hi = __reduce_max_sync(0xffffffffu, c_hi);
@@ -651,7 +646,6 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
             float tc = 1.0f, ts = 0.0f;
             if (a.fdem > 0.0f) sincosf(a.two_pi_f * tau, &ts, &tc);
             if (!isinf(tau)) ph = make_float2(tw * tc, tw * ts);
-            if (isnan(tau - a.t0)) tau = NAN;
           }
           tab_w[(e - c0) * kPx + pl] = ph;
           tab_t[(e - c0) * kPx + pl] = tau;
@@ -664,14 +658,7 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
 #pragma unroll 1
       for (int e = 0; e < n_ev; ++e, trace += ev_stride) {
         const float tau = tab_t[e * kPx + pl];
-        if (!(fabsf(tau) < INFINITY)) {
-          // A delay that is no number makes the channels' samples so, as the
-          // interpolation of das_fast_kernel does (its index converts to 0).
-          if (isnan(tau))
-#pragma unroll
-            for (int k = 0; k < kG; ++k) acc[k] = make_float2(NAN, NAN);
-          continue;
-        }
+        if (isinf(tau)) continue;
         const float2 w2 = tab_w[e * kPx + pl];
         const float2 tau2 = make_float2(tau, tau), wr2 = make_float2(w2.x, w2.x);
         // Every load of the group is issued before the first is used; an
