@@ -175,8 +175,8 @@ int usx_cu_bf_variant_order(int index, int* deep_first);
  * tile_lines is the CTA's pixel warps, 32 x tile_lines pixels).
  * Families 1-4 fall back to variant 0 where they do not apply (RF data,
  * incoherent compounding, and for family 4 traces of one sample or of more
- * than 2^23; families 1 and 3 also need plane waves, family 2
- * at most 256 channels). */
+ * than 2^23, or a transmit or time origin that is not finite; families 1 and 3
+ * also need plane waves, family 2 at most 256 channels). */
 int usx_cu_bf_variant_kind(int index, int* kind);
 int usx_cu_bf_plan_set_variant(usx_bf_plan* plan, int index);
 int usx_cu_bf_plan_get_variant(const usx_bf_plan* plan, int* index);

@@ -70,3 +70,62 @@ def test_demodulation_of_the_longest_traces(gpu, oracle, n_smp, taps):
     iq = torch.full(want.shape, float("nan"), dtype=torch.complex64, device="cuda")
     ctx.demodulate(ch, capi.demod_config(filter_taps=taps), d.data_ptr(), iq.data_ptr())
     assert np.abs(iq.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()
+
+
+def probe_channel(capi, n_ev, n_el=40, n_smp=260, kind=1, t0=0.0, iq=True):
+    tx = [dict(type=kind, angle=0.1 * e - 0.1, focus=(0.0, 0.0, -0.01 - 1e-3 * e), delays=np.zeros(n_el, np.float32),
+               apodization=np.ones(n_el, np.float32)) for e in range(n_ev)]
+    return tx, lambda: capi.Channel(capi.Probe(n_el, 3e-4, 2.7e-4, 5e-3, 5e6, 0.6), capi.Medium(1540.0, 0.5, 1000.0),
+                                    capi.Acquisition(2e7, n_smp, t0, 5e3), tx, iq, 5e6 if iq else 0.0)
+
+
+def image_points(n0=9, n1=20):
+    ax0 = np.linspace(-5e-3, 5e-3, n0).astype(np.float32)
+    ax1 = np.linspace(0.0, 9e-3, n1).astype(np.float32)
+    pts = np.stack(np.broadcast_arrays(ax0[:, None], 0.0, ax1[None]), -1).astype(np.float32)
+    return ax0, ax1, pts.reshape(-1, 3).copy()
+
+
+def frames_of(capi, torch, ctx, ch, grid, data, variants, mv=False, **cfg):
+    d = torch.from_numpy(data).cuda()
+    out, got = torch.empty(grid.shape, dtype=torch.complex64, device="cuda"), []
+    for v in variants:
+        plan = ctx.plan(ch, grid, capi.bf_config(f_number=1.0, combiner=2 if mv else 0, **cfg))
+        if mv:
+            plan.set_mv_mode(3)
+        if v is not None:
+            plan.set_variant(v)
+        out.fill_(7.0)
+        plan.execute(d.data_ptr(), out.data_ptr())
+        got.append(out.cpu().numpy())
+        plan.close()
+    return got
+
+
+@pytest.mark.parametrize("mv", [False, True])
+@pytest.mark.parametrize("what", ["angle", "focus", "t0", "late t0", "points"])
+@pytest.mark.parametrize("weighting", [0, 1])
+def test_delays_that_are_no_numbers_reach_the_frame(gpu, what, weighting, mv):
+    """A NaN in an event's steering, in the time origin or in a point is not
+    dropped: each channel-warp shape gives the pixels of the thread-per-pixel
+    kernel, NaN where its are."""
+    torch, capi, ctx = gpu
+    t0 = np.nan if what == "t0" else np.inf if what == "late t0" else 0.0
+    tx, channel = probe_channel(capi, 3, kind=2 if what == "focus" else 1, t0=t0)
+    if what == "angle":
+        tx[1]["angle"] = np.nan
+    if what == "focus":
+        tx[2]["focus"] = (0.0, np.nan, -0.01)
+    ax0, ax1, pts = image_points()
+    if what == "points":
+        for k, c in ((30, 0), (75, 1), (120, 2), (50, 0), (95, 1), (140, 2)):
+            pts[k, c] = np.nan if k in (30, 75, 120) else np.inf
+        pts[170] = (0.5 * 3e-4, 0.0, np.nan)   # over an element
+    rng = np.random.default_rng(8)
+    iq = (rng.normal(size=(3, 40, 260)) + 1j * rng.normal(size=(3, 40, 260))).astype(np.complex64)
+    got = frames_of(capi, torch, ctx, channel(), capi.Grid(0, ax0, ax1, pts), iq, (0, None, 1, 2, 3, 22, 23), mv=mv,
+                    transmit_weighting=weighting, rx_window=0)
+    if not mv and what not in ("late t0",):
+        assert np.isnan(got[0]).any()
+    for g in got[1:]:
+        assert np.array_equal(g, got[0], equal_nan=True)

@@ -497,8 +497,11 @@ __host__ __device__ constexpr size_t exp_smem_bytes(int events, int pixel_warps,
 // Sample indices take floor(idx) by one directed-rounding addition: 2^23 + idx
 // rounded down is 2^23 + floor(idx) for 0 <= idx < 2^23, its low mantissa bits
 // the integer (no conversion instruction, which run at a fraction of the FP32
-// rate). A negative, infinite or NaN index, or one of 2^23 and above, gives at
-// least 2^23: past every trace these kernels take.
+// rate). A negative or infinite index, or one of 2^23 and above, gives at least
+// 2^23: past every trace these kernels take. So does NaN, where das_fast_kernel
+// reads sample 0 and shows the NaN: a point's coordinate that is no number
+// reaches the frame through the receive phasor, and plans whose events' delays
+// may be none (finite_transmit) do not come here.
 constexpr int kMaxFastSamples = 1 << 23;
 
 template <int kG, int kPW, int kCQ, int kWL, int kTL, bool kSum>
@@ -1791,6 +1794,15 @@ size_t channel_warp_smem(const DasVariant& v, int events, bool sum, int* tab_eve
 // directed-rounding addition; a pair load needs two samples).
 bool channel_warp_samples(int n_smp) { return n_smp >= 2 && n_smp <= kMaxFastSamples; }
 
+// Whether a transmit's delays are numbers at every finite point. The
+// channel-warp kernels drop an event whose sample index is not a number, where
+// das_fast_kernel's index converts to 0 and the frame shows the NaN.
+bool finite_transmit(const TxDev& t) {
+  for (float v : {t.ox, t.sin_a, t.cos_a, t.fx, t.fy, t.fz, t.axis_len, t.dx, t.dy, t.dz, t.d_origin_focus})
+    if (!std::isfinite(v)) return false;
+  return true;
+}
+
 // The shape of a plan whose variant was neither set nor tuned (IQ, coherent or
 // select). Measured at 128 channels (us; shapes by index):
 //   at most one 32-pixel tile per SM: all channels at once (3), the rest wait
@@ -2025,6 +2037,7 @@ struct usx_bf_plan {
   int das_variant = 0;         // index into kDasVariants (set by the caller or the autotuner)
   bool variant_set = false;    // false: default_variant's rule picks the shape
   bool all_plane_waves = false;  // every event is a plane wave (the staged kernel's bound)
+  bool finite_delays = false;    // every number the delays are formed from is finite (finite_transmit)
   int* d_mv_stats = nullptr;   // [0] FP64 re-solves, [1] factorisation failures, [2] learned-MV gate rejections
   // Learned minimum variance: the network (not owned) and the gate on |1^H w - 1|.
   usx_mlp* mlp = nullptr;
@@ -2170,7 +2183,7 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
   const DasVariant* dvp = &kDasVariants[!plan->variant_set && plain_iq
                                             ? default_variant(plan->n0, plan->n1, n_frames, ev_per_frame, ctx->sm_count)
                                             : plan->das_variant];
-  if (dvp->channel_warps > 1 && !channel_warp_samples(a.n_smp)) dvp = &kDasVariants[0];
+  if (dvp->channel_warps > 1 && !(channel_warp_samples(a.n_smp) && plan->finite_delays)) dvp = &kDasVariants[0];
   if (dvp->staged) {
     const bool ok = plan->cd.is_iq && plan->all_plane_waves && a.compounding != USX_COMP_INCOHERENT &&
                     reinterpret_cast<uintptr_t>(data) % 16 == 0 && a.n_smp >= kStageW + 2;
@@ -2479,6 +2492,9 @@ int usx_cu_bf_plan_create(usx_ctx* ctx, const usx_channel_desc* cd, const usx_gr
   for (int e = 0; e < n_ev; ++e) txs[static_cast<size_t>(e)] = make_txdev(cd->probe, cd->transmits[e]);
   p->all_plane_waves = n_ev > 0;
   for (int e = 0; e < n_ev; ++e) p->all_plane_waves = p->all_plane_waves && txs[static_cast<size_t>(e)].type == USX_TX_PLANE_WAVE;
+  p->finite_delays = std::isfinite(cd->acq.t0) && std::isfinite(cd->acq.sampling_frequency) &&
+                     std::isfinite(cd->medium.speed_of_sound);
+  for (const TxDev& t : txs) p->finite_delays = p->finite_delays && finite_transmit(t);
   cudaError_t e1 = cudaMalloc(&p->d_points, sizeof(float) * 3 * n_pix);
   cudaError_t e2 = cudaMalloc(&p->d_tx, sizeof(TxDev) * std::max(1, n_ev));
   cudaError_t e3 = cudaMalloc(&p->d_mv_stats, sizeof(int) * 4);
@@ -2761,7 +2777,8 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     int tab_events = 1;
     // Traces the channel-warp body does not take go to das_fast_kernel's tiles.
     bool cw = iq;
-    for (int k = 0; k < m; ++k) cw = cw && channel_warp_samples(plans[i0 + k]->cd.acq.n_samples);
+    for (int k = 0; k < m; ++k)
+      cw = cw && channel_warp_samples(plans[i0 + k]->cd.acq.n_samples) && plans[i0 + k]->finite_delays;
     for (int k = 0; k < m; ++k) {
       const usx_bf_plan* p = plans[i0 + k];
       BfArgs a = make_args(p);
