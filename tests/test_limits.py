@@ -129,3 +129,38 @@ def test_delays_that_are_no_numbers_reach_the_frame(gpu, what, weighting, mv):
         assert np.isnan(got[0]).any()
     for g in got[1:]:
         assert np.array_equal(g, got[0], equal_nan=True)
+
+
+@pytest.mark.parametrize("n_ev,n_el", [(1, 40), (2, 9), (5, 64), (40, 24), (90, 40)])
+@pytest.mark.parametrize("mv", [False, True])
+def test_selected_events_are_the_first_of_the_largest_weight(gpu, n_ev, n_el, mv):
+    """Beams in pairs of equal illumination: the pixels take the first of a
+    pair, in every shape as in the thread-per-pixel kernel, in a queue too."""
+    torch, capi, ctx = gpu
+    pitch, n_smp = 3e-4, 260
+    pos = (np.arange(n_el) - 0.5 * (n_el - 1)) * pitch
+    tx = []
+    for e in range(n_ev):
+        x = 0.8 * pos[-1] * (2.0 * (e // 2) / max(1, (n_ev + 1) // 2 - 1) - 1.0) if n_ev > 2 else 0.0
+        apod = (np.abs(pos - x) <= 6 * pitch).astype(np.float32)
+        tx.append(dict(type=0, angle=0.0, focus=(x, 0.0, 0.006), origin=(x, 0.0, 0.0),
+                       delays=np.zeros(n_el, np.float32), apodization=apod))
+    ch = capi.Channel(capi.Probe(n_el, pitch, 2.7e-4, 5e-3, 5e6, 0.6), capi.Medium(1540.0, 0.5, 1000.0),
+                      capi.Acquisition(2e7, n_smp, 0.0, 5e3), tx, True, 5e6)
+    grid = capi.Grid(0, *image_points(13, 37))
+    rng = np.random.default_rng(n_ev)
+    iq = (rng.normal(size=(n_ev, n_el, n_smp)) + 1j * rng.normal(size=(n_ev, n_el, n_smp))).astype(np.complex64)
+    got = frames_of(capi, torch, ctx, ch, grid, iq, (0, None, 1, 2, 3, 22, 23), mv=mv, compounding=2)
+    assert np.abs(got[0]).max() > 0
+    for g in got[1:]:
+        assert np.array_equal(g, got[0])
+    if not mv:
+        plans = [ctx.plan(ch, grid, capi.bf_config(f_number=1.0, compounding=c)) for c in (2, 0, 2)]
+        d = torch.from_numpy(iq).cuda()
+        out = torch.full((3, *grid.shape), 7.0, dtype=torch.complex64, device="cuda")
+        ctx.execute_queue(plans, [d.data_ptr()] * 3, [o.data_ptr() for o in out])
+        want = frames_of(capi, torch, ctx, ch, grid, iq, (0,))[0]
+        for o, w in zip(out.cpu().numpy(), (got[0], want, got[0])):
+            assert np.array_equal(o, w)
+        for p in plans:
+            p.close()

@@ -484,6 +484,13 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_fast_kernel(const B
 // 0.175, (4,4,4,4,4) 3.85 / 0.179 (its 75-event table leaves one CTA per SM).
 // Before the last step: (4,2,8,2,2) 2.82 / 0.236, (2,2,8,4,8) 2.74 / 0.225, 8
 // channels per group 4.5 / 0.319, 40 registers with three CTAs 3.5 / 0.226.
+//
+// Select compounding has instances of its own (kSel): a pixel sums one event, so
+// the channel warps share the search for it, the table holds that event alone
+// and the event loop runs once. (16 channels, 256 x 640 pixels, 100
+// events: 99 us; 451 with each channel warp searching all events and every pixel
+// stepping over the others' entries; das_fast_kernel 184.) The other instances keep their branches for it, which they never take: without
+// them the compiler schedules the 75-event frame to 2.93 ms.
 constexpr int kTabEvents = 80;   // events a CTA tabulates at once (more go in chunks)
 
 // Dynamic shared memory of the channel-warp kernels: the transmit table of
@@ -504,7 +511,7 @@ __host__ __device__ constexpr size_t exp_smem_bytes(int events, int pixel_warps,
 // may be none (finite_transmit) do not come here.
 constexpr int kMaxFastSamples = 1 << 23;
 
-template <int kG, int kPW, int kCQ, int kWL, int kTL, bool kSum>
+template <int kG, int kPW, int kCQ, int kWL, int kTL, bool kSum, bool kSel>
 __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long frame) {
   constexpr int kTD = 32 * kPW / kTL, kWD = 32 / kWL, kWarpCols = kTD / kWD;
   static_assert(32 % kWL == 0 && kTL % kWL == 0 && kTD % kWD == 0 && kG % 2 == 0, "warp shape must tile the CTA");
@@ -547,7 +554,7 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
   int best_ev = -1;
   float best_w = 0.0f;
   if (select && valid) {
-    for (int ev = ev_lo; ev < ev_hi; ++ev) {
+    for (int ev = kSel ? ev_lo + cq : ev_lo; ev < ev_hi; ev += kSel ? kCQ : 1) {
       const float tw = tx_sensitivity_fast(a.tx[ev], px, pz, a.lambda);
       if (tw > best_w) {
         best_w = tw;
@@ -555,6 +562,8 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
       }
     }
   }
+  // The channel warps share the search, through the table's space.
+  if (kSel && select) tab_w[cq * kPx + pl] = make_float2(best_w, __int_as_float(best_ev));
   const float2* iq = a.iq + frame * a.data_stride;
   const unsigned n_last = static_cast<unsigned>(a.n_smp - 1);
   const long ev_stride = static_cast<long>(a.n_ch) * a.n_smp;
@@ -570,6 +579,16 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
     s_range[1] = -1;
   }
   __syncthreads();   // (also: the previous tile's shared memory is no longer read)
+  if (kSel && select)   // the first event of the largest weight
+#pragma unroll 1
+    for (int q = 0; q < kCQ; ++q) {
+      const float2 v = tab_w[q * kPx + pl];
+      const int ev = __float_as_int(v.y);
+      if (v.x > best_w || (v.x == best_w && v.x > 0.0f && ev < best_ev)) {
+        best_w = v.x;
+        best_ev = ev;
+      }
+    }
   if (cq == 0) {
     int c_lo = a.n_ch, c_hi = -1;
     if (valid && pz > 0.0f) {
@@ -597,6 +616,11 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
         a.y_out[(frame * a.n_pix + pix) * a.n_ch + ch] = make_float2(0.f, 0.f);
     }
 
+  // Select: each pixel's own event is the only one, entry ev_lo of the table.
+  if (kSel && select) {
+    ev_hi = ev_lo + 1;
+    iq += (max(best_ev, ev_lo) - ev_lo) * ev_stride;
+  }
   const bool one_chunk = ev_hi - ev_lo <= a.tab_events;
   for (int g0 = g_lo; g0 < g_hi; g0 += kCQ) {
     const int grp = g0 + cq, g = grp * kG;
@@ -632,12 +656,12 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
         // infinite), which puts every sample index past the trace.
         if (!one_chunk) __syncthreads();
         for (int e = c0 + cq; e < c1; e += kCQ) {
-          const TxDev& t = a.tx[e];
+          const TxDev& t = a.tx[kSel && select ? max(best_ev, ev_lo) : e];
           float tw;
           if (!valid)
             tw = 0.0f;
           else if (select)
-            tw = (best_ev == e && best_w > 0.0f) ? 1.0f : 0.0f;
+            tw = ((kSel || best_ev == e) && best_w > 0.0f) ? 1.0f : 0.0f;
           else if (a.tx_weighting)
             tw = tx_sensitivity_fast(t, px, pz, a.lambda);
           else
@@ -788,14 +812,14 @@ __device__ __forceinline__ void das_export_body(const BfArgs& a, int tile, long 
   }
 }
 
-template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB>
+template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB, bool kSel>
 __global__ void __launch_bounds__(32 * kPW * kCQ, MB) das_export_kernel(const BfArgs a) {
-  das_export_body<kG, kPW, kCQ, kWL, kTL, false>(a, blockIdx.x, blockIdx.y);
+  das_export_body<kG, kPW, kCQ, kWL, kTL, false, kSel>(a, blockIdx.x, blockIdx.y);
 }
 // The channel-combining instance (delay-and-sum, DMAS, coherence factor).
-template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB>
+template <int kG, int kPW, int kCQ, int kWL, int kTL, int MB, bool kSel>
 __global__ void __launch_bounds__(32 * kPW * kCQ, MB) das_csum_kernel(const BfArgs a) {
-  das_export_body<kG, kPW, kCQ, kWL, kTL, true>(a, blockIdx.x, blockIdx.y);
+  das_export_body<kG, kPW, kCQ, kWL, kTL, true, kSel>(a, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------------------
@@ -837,6 +861,7 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_queue_kernel(const 
 
 // The same queue over das_csum_kernel's body (IQ plans): CTAs of 2 pixel
 // warps x 8 channel warps on 8-line x 8-depth tiles.
+template <bool kSel>   // some entry compounds by selection
 __global__ void __launch_bounds__(512, 2) das_csum_queue_kernel(const DasQueueArgs q) {
   __shared__ int s_item;
   const int total = q.first[q.n];
@@ -850,7 +875,7 @@ __global__ void __launch_bounds__(512, 2) das_csum_queue_kernel(const DasQueueAr
     while (e + 1 < q.n && item >= q.first[e + 1]) ++e;
     const int local = item - q.first[e];
     const int frame = local / q.tiles[e], tile = local - frame * q.tiles[e];
-    das_export_body<4, 2, 8, 4, 8, true>(q.args[e], tile, frame);
+    das_export_body<4, 2, 8, 4, 8, true, kSel>(q.args[e], tile, frame);
   }
 }
 
@@ -1739,6 +1764,8 @@ struct DasVariant {
   int producer_warps = 0;   // das_ring_kernel: one warp beside the tile's warps
   int channel_warps = 1;    // das_export_kernel: warps per pixel warp (IQ: MV exports, coherent sums; else variant 0)
   void (*sum)(BfArgs) = nullptr;   // das_csum_kernel, the channel-combining instance (plain IQ launches)
+  void (*iq_select)(BfArgs) = nullptr;    // the channel-warp kernels' instances for select compounding
+  void (*sum_select)(BfArgs) = nullptr;
   int grid_lines = 0;       // das_export_kernel: lines of the tile (32 x pixel warps / grid_lines depths)
 };
 // RF input (the reference's interp_rf path) keeps the default shape in
@@ -1762,8 +1789,9 @@ constexpr DasVariant das_staged_variant() {
 // launches use variant 0.
 template <int G, int PW, int CQ, int WL, int TL, int MB>
 constexpr DasVariant das_export_variant() {
-  return DasVariant{G, PW, 0, WL, false, das_export_kernel<G, PW, CQ, WL, TL, MB>, das_fast_kernel<false, 16, 4, 1>,
-                    false, false, 0, CQ, das_csum_kernel<G, PW, CQ, WL, TL, MB>, TL};
+  return DasVariant{G, PW, 0, WL, false, das_export_kernel<G, PW, CQ, WL, TL, MB, false>, das_fast_kernel<false, 16, 4, 1>,
+                    false, false, 0, CQ, das_csum_kernel<G, PW, CQ, WL, TL, MB, false>,
+                    das_export_kernel<G, PW, CQ, WL, TL, MB, true>, das_csum_kernel<G, PW, CQ, WL, TL, MB, true>, TL};
 }
 // The producer-warp ring (same applicability as the staged kernel).
 template <int G, int TL, int S>
@@ -1786,8 +1814,9 @@ constexpr int kNumDasVariants = static_cast<int>(sizeof(kDasVariants) / sizeof(k
 
 // Dynamic shared memory of a channel-warp launch whose frames have `events`
 // events each, and the events its table holds.
-size_t channel_warp_smem(const DasVariant& v, int events, bool sum, int* tab_events) {
-  *tab_events = std::max(1, std::min(events, kTabEvents));
+// (Select: one event, and room for the channel warps' candidates.)
+size_t channel_warp_smem(const DasVariant& v, int events, bool select, bool sum, int* tab_events) {
+  *tab_events = select ? v.channel_warps : std::max(1, std::min(events, kTabEvents));
   return exp_smem_bytes(*tab_events, v.tile_lines, v.channel_warps, v.group, sum);
 }
 // The channel-warp kernels take traces of 2 to 2^23 samples (floor by a
@@ -2213,9 +2242,10 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
     prof_begin(ctx, csum ? "das_csum_kernel" : cexport ? "das_export_kernel(mv export)" : name);
     if (csum) {
       BfArgs t = b;
-      const size_t tb = channel_warp_smem(dv, ev_per_launch, true, &t.tab_events);
-      if (int rc_ = smem_limit(reinterpret_cast<const void*>(dv.sum), tb)) return rc_;
-      dv.sum<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
+      const size_t tb = channel_warp_smem(dv, ev_per_launch, b.compounding == USX_COMP_SELECT, true, &t.tab_events);
+      auto kern = b.compounding == USX_COMP_SELECT ? dv.sum_select : dv.sum;
+      if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), tb)) return rc_;
+      kern<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
     } else if (fast && dv.channel_warps > 1 && !(b.is_mv && plan->cd.is_iq)) {
       // A channel-warp shape on an RF or incoherent launch: variant 0.
       const DasVariant& d0 = kDasVariants[0];
@@ -2226,9 +2256,10 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
         d0.rf<<<g0, 32 * d0.tile_lines, 0, ctx->stream>>>(b);
     } else if (fast && dv.channel_warps > 1) {
       BfArgs t = b;
-      const size_t tb = channel_warp_smem(dv, ev_per_launch, false, &t.tab_events);
-      if (int rc_ = smem_limit(reinterpret_cast<const void*>(dv.iq), tb)) return rc_;
-      dv.iq<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
+      const size_t tb = channel_warp_smem(dv, ev_per_launch, b.compounding == USX_COMP_SELECT, false, &t.tab_events);
+      auto kern = b.compounding == USX_COMP_SELECT ? dv.iq_select : dv.iq;
+      if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), tb)) return rc_;
+      kern<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
     } else if (table) {
       dv.iq<<<grid_das, 32 * table_warps(dv.group, b.n_ch), table_smem, ctx->stream>>>(b);
     } else if (fast) {
@@ -2776,7 +2807,7 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     q.first[0] = 0;
     int tab_events = 1;
     // Traces the channel-warp body does not take go to das_fast_kernel's tiles.
-    bool cw = iq;
+    bool cw = iq, any_select = false;
     for (int k = 0; k < m; ++k)
       cw = cw && channel_warp_samples(plans[i0 + k]->cd.acq.n_samples) && plans[i0 + k]->finite_delays;
     for (int k = 0; k < m; ++k) {
@@ -2795,7 +2826,9 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
       }
       const int tiles = cw ? ceil_div(p->n0, 8) * ceil_div(p->n1, 8) : ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
       q.args[q.n] = a;
-      tab_events = std::max(tab_events, std::min(kTabEvents, a.ev_end - a.ev_begin));
+      any_select = any_select || a.compounding == USX_COMP_SELECT;
+      tab_events = std::max(tab_events, a.compounding == USX_COMP_SELECT ? 8   // (its channel warps)
+                                                                         : std::min(kTabEvents, a.ev_end - a.ev_begin));
       q.tiles[q.n] = tiles;
       q.first[q.n + 1] = q.first[q.n] + tiles;
       ++q.n;
@@ -2805,7 +2838,8 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     USX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream));
     // IQ: das_csum_kernel's body (2 pixel warps x 8 channel warps); RF, and
     // traces that body does not take: das_fast_kernel's shape.
-    const void* kern = cw   ? reinterpret_cast<const void*>(das_csum_queue_kernel)
+    auto* csum_queue = any_select ? das_csum_queue_kernel<true> : das_csum_queue_kernel<false>;
+    const void* kern = cw   ? reinterpret_cast<const void*>(csum_queue)
                        : iq ? reinterpret_cast<const void*>(das_queue_kernel<true, 16, 4, 1>)
                             : reinterpret_cast<const void*>(das_queue_kernel<false, 16, 4, 1>);
     const int threads = cw ? 512 : 32 * 4;
@@ -2818,7 +2852,7 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     const unsigned grid = static_cast<unsigned>(std::max(1, per_sm) * ctx->sm_count);
     prof_begin(ctx, cw ? "das_csum_queue_kernel" : "das_queue_kernel");
     if (cw)
-      das_csum_queue_kernel<<<grid, threads, tb, ctx->stream>>>(q);
+      csum_queue<<<grid, threads, tb, ctx->stream>>>(q);
     else if (iq)
       das_queue_kernel<true, 16, 4, 1><<<grid, threads, 0, ctx->stream>>>(q);
     else
