@@ -131,6 +131,44 @@ def test_delays_that_are_no_numbers_reach_the_frame(gpu, what, weighting, mv):
         assert np.array_equal(g, got[0], equal_nan=True)
 
 
+@pytest.mark.parametrize("cfg", [{}, dict(compounding=1), dict(compounding=2)])
+def test_rf_frames_are_the_same_in_every_shape(gpu, cfg):
+    """RF data run one launch shape whichever is set, and tuning picks one."""
+    torch, capi, ctx = gpu
+    _, channel = probe_channel(capi, 3, iq=False)
+    grid = capi.Grid(0, *image_points())
+    rf = np.random.default_rng(9).normal(size=(3, 40, 260)).astype(np.float32)
+    n = len(capi.das_variants())
+    got = frames_of(capi, torch, ctx, channel(), grid, rf, (None, *range(n)), **cfg)
+    assert np.abs(got[0]).max() > 0 and not (got[0] == 7.0).any()
+    for v, g in enumerate(got[1:]):
+        assert np.array_equal(g, got[0]), v
+    plan = ctx.plan(channel(), grid, capi.bf_config(f_number=1.0, **cfg))
+    d, out = torch.from_numpy(rf).cuda(), torch.full(grid.shape, 7.0, dtype=torch.complex64, device="cuda")
+    best, ms = plan.autotune(d.data_ptr(), out.data_ptr(), 1)
+    assert 0 <= best < n and all(m > 0 for m in ms)
+    assert np.array_equal(out.cpu().numpy(), got[0])
+    plan.close()
+
+
+def test_a_first_large_rf_frame_is_tuned(gpu):
+    """The host class times the shapes on a plan's first frame of 1e9 pixel x
+    event x channel terms or more: RF as IQ, the frame that of the next call."""
+    import usx
+    probe = usx.presets.linear_5mhz()
+    probe.n_elements = 32
+    acq = usx.presets.acquisition(probe, depth=0.02, medium=usx.Medium(), samples_per_wavelength=4.0)
+    cfg = usx.SimulatorConfig()
+    cfg.noise_db = -200.0
+    sim = usx.Simulator(probe, usx.Medium(), acq, cfg)
+    raw = sim.simulate(sim.make_plane_waves(usx.angles_deg(-6, 6, 31)), usx.Phantom.speckle_box(-0.004, 0.004, 0.004, 0.018,
+                                                                                               0.0, 100, 5))
+    grid = usx.ScanGrid.cartesian(-0.004, 0.004, 800, 0.004, 0.018, 1300)
+    bf = usx.Beamformer(usx.BeamformerConfig())
+    first, second = (np.asarray(bf.beamform(raw, grid).data) for _ in range(2))
+    assert np.abs(first).max() > 0 and np.array_equal(first, second)
+
+
 @pytest.mark.parametrize("n_ev,n_el", [(1, 40), (2, 9), (5, 64), (40, 24), (90, 40)])
 @pytest.mark.parametrize("mv", [False, True])
 def test_selected_events_are_the_first_of_the_largest_weight(gpu, n_ev, n_el, mv):

@@ -489,8 +489,9 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_fast_kernel(const B
 // the channel warps share the search for it, the table holds that event alone
 // and the event loop runs once. (16 channels, 256 x 640 pixels, 100
 // events: 99 us; 451 with each channel warp searching all events and every pixel
-// stepping over the others' entries; das_fast_kernel 184.) The other instances keep their branches for it, which they never take: without
-// them the compiler schedules the 75-event frame to 2.93 ms.
+// stepping over the others' entries; das_fast_kernel 184.) The other instances
+// keep their branches for it, which they never take: without them the compiler
+// schedules the 75-event frame to 2.93 ms.
 constexpr int kTabEvents = 80;   // events a CTA tabulates at once (more go in chunks)
 
 // Dynamic shared memory of the channel-warp kernels: the transmit table of
@@ -2212,6 +2213,7 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
   const DasVariant* dvp = &kDasVariants[!plan->variant_set && plain_iq
                                             ? default_variant(plan->n0, plan->n1, n_frames, ev_per_frame, ctx->sm_count)
                                             : plan->das_variant];
+  if (!plan->cd.is_iq) dvp = &kDasVariants[0];   // RF has one launch shape
   if (dvp->channel_warps > 1 && !(channel_warp_samples(a.n_smp) && plan->finite_delays)) dvp = &kDasVariants[0];
   if (dvp->staged) {
     const bool ok = plan->cd.is_iq && plan->all_plane_waves && a.compounding != USX_COMP_INCOHERENT &&
@@ -2246,14 +2248,11 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
       auto kern = b.compounding == USX_COMP_SELECT ? dv.sum_select : dv.sum;
       if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), tb)) return rc_;
       kern<<<grid_das, 32 * dv.tile_lines * dv.channel_warps, tb, ctx->stream>>>(t);
-    } else if (fast && dv.channel_warps > 1 && !(b.is_mv && plan->cd.is_iq)) {
-      // A channel-warp shape on an RF or incoherent launch: variant 0.
+    } else if (fast && dv.channel_warps > 1 && !b.is_mv) {
+      // A channel-warp shape on an incoherent launch: variant 0.
       const DasVariant& d0 = kDasVariants[0];
       const dim3 g0(ceil_div(plan->n0, d0.tile_lines) * ceil_div(plan->n1, 32), grid_das.y);
-      if (plan->cd.is_iq)
-        d0.iq<<<g0, 32 * d0.tile_lines, 0, ctx->stream>>>(b);
-      else
-        d0.rf<<<g0, 32 * d0.tile_lines, 0, ctx->stream>>>(b);
+      d0.iq<<<g0, 32 * d0.tile_lines, 0, ctx->stream>>>(b);
     } else if (fast && dv.channel_warps > 1) {
       BfArgs t = b;
       const size_t tb = channel_warp_smem(dv, ev_per_launch, b.compounding == USX_COMP_SELECT, false, &t.tab_events);
