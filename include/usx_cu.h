@@ -152,10 +152,10 @@ int usx_cu_bf_plan_set_precision(usx_bf_plan* plan, int precision);
  * variant (plus a warm-up) `repeats` times, keeps the fastest in the plan,
  * writes every variant's mean milliseconds to ms_out[variant] (host, may be
  * NULL; usx_cu_bf_variant_count() entries), leaves the frame of the chosen
- * variant in `frame` and synchronises. A plan whose variant was neither set
- * nor tuned reports 0; its IQ frames (coherent or select) take the
- * channel-warp shape that a rule on pixels and events picks, its others
- * variant 0. */
+ * variant in `frame` and synchronises. The IQ frames (coherent or select) of
+ * a plan whose variant was neither set nor tuned take the shape that a rule on
+ * pixels, frames and events picks, its others variant 0; get_variant gives the
+ * shape of one acquisition. */
 int usx_cu_bf_variant_count(void);
 int usx_cu_bf_variant_info(int index, int* channel_group, int* tile_lines, int* min_blocks, int* warp_lines);
 /* The order in which variant i dispatches its CTA tiles: *deep_first = 1 when

@@ -202,3 +202,23 @@ def test_selected_events_are_the_first_of_the_largest_weight(gpu, n_ev, n_el, mv
             assert np.array_equal(o, w)
         for p in plans:
             p.close()
+
+
+@pytest.mark.parametrize("n0,n1,n_ev", [(4, 8, 3), (40, 90, 3), (300, 400, 3), (300, 400, 20), (200, 300, 70)])
+def test_a_plan_reports_the_shape_it_runs(gpu, n0, n1, n_ev):
+    """Neither set nor tuned: the shape of one acquisition, so that what is
+    read from a plan and set on another leaves its speed as it was."""
+    torch, capi, ctx = gpu
+    _, channel = probe_channel(capi, n_ev)
+    grid = capi.Grid(0, *image_points(n0, n1))
+    kinds = [v[5] for v in capi.das_variants()]
+    for cfg, iq, want in ((dict(), True, 4), (dict(compounding=2), True, 4), (dict(compounding=1), True, 0)):
+        plan = ctx.plan(channel(), grid, capi.bf_config(f_number=1.0, **cfg))
+        assert kinds[plan.variant()] == want
+        plan.set_variant(0)
+        assert plan.variant() == 0
+        plan.close()
+    _, rf = probe_channel(capi, n_ev, iq=False)
+    plan = ctx.plan(rf(), grid, capi.bf_config(f_number=1.0))
+    assert plan.variant() == 0
+    plan.close()

@@ -2185,6 +2185,17 @@ BfArgs make_args(const usx_bf_plan* p) {
 }
 
 
+// Whether the channel-warp kernels take the plan's traces and delays.
+bool channel_warp_plan(const usx_bf_plan* p) { return channel_warp_samples(p->cd.acq.n_samples) && p->finite_delays; }
+
+// The launch shape of a call of n_frames frames of `events` events each: the
+// plan's, or the rule's where none was set or tuned.
+int plan_variant(const usx_bf_plan* p, int n_frames, int events) {
+  if (p->variant_set || !p->cd.is_iq || p->cfg.compounding == USX_COMP_INCOHERENT || !channel_warp_plan(p) || events <= 0)
+    return p->das_variant;
+  return default_variant(p->n0, p->n1, n_frames, events, p->ctx->sm_count);
+}
+
 int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_stride,
                float* frames, int64_t frame_stride, int seq_epf) {
   if (!plan || !data || !frames) return fail(USX_ERR_INVALID, "usx_cu_bf_execute: null argument");
@@ -2209,12 +2220,9 @@ int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_s
     return USX_OK;
   }
   const bool fast = plan->precision == USX_BF_FAST;
-  const bool plain_iq = plan->cd.is_iq && a.compounding != USX_COMP_INCOHERENT;
-  const DasVariant* dvp = &kDasVariants[!plan->variant_set && plain_iq
-                                            ? default_variant(plan->n0, plan->n1, n_frames, ev_per_frame, ctx->sm_count)
-                                            : plan->das_variant];
+  const DasVariant* dvp = &kDasVariants[plan_variant(plan, n_frames, ev_per_frame)];
   if (!plan->cd.is_iq) dvp = &kDasVariants[0];   // RF has one launch shape
-  if (dvp->channel_warps > 1 && !(channel_warp_samples(a.n_smp) && plan->finite_delays)) dvp = &kDasVariants[0];
+  if (dvp->channel_warps > 1 && !channel_warp_plan(plan)) dvp = &kDasVariants[0];
   if (dvp->staged) {
     const bool ok = plan->cd.is_iq && plan->all_plane_waves && a.compounding != USX_COMP_INCOHERENT &&
                     reinterpret_cast<uintptr_t>(data) % 16 == 0 && a.n_smp >= kStageW + 2;
@@ -2634,7 +2642,7 @@ int usx_cu_bf_plan_set_variant(usx_bf_plan* plan, int index) {
 
 int usx_cu_bf_plan_get_variant(const usx_bf_plan* plan, int* index) {
   if (!plan || !index) return fail(USX_ERR_INVALID, "usx_cu_bf_plan_get_variant: null argument");
-  *index = plan->das_variant;
+  *index = plan_variant(plan, 1, plan->ev_end - plan->ev_begin);
   return USX_OK;
 }
 
@@ -2805,10 +2813,9 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     q.n = 0;
     q.first[0] = 0;
     int tab_events = 1;
-    // Traces the channel-warp body does not take go to das_fast_kernel's tiles.
+    // Plans the channel-warp body does not take go to das_fast_kernel's tiles.
     bool cw = iq, any_select = false;
-    for (int k = 0; k < m; ++k)
-      cw = cw && channel_warp_samples(plans[i0 + k]->cd.acq.n_samples) && plans[i0 + k]->finite_delays;
+    for (int k = 0; k < m; ++k) cw = cw && channel_warp_plan(plans[i0 + k]);
     for (int k = 0; k < m; ++k) {
       const usx_bf_plan* p = plans[i0 + k];
       BfArgs a = make_args(p);
