@@ -222,3 +222,22 @@ def test_a_plan_reports_the_shape_it_runs(gpu, n0, n1, n_ev):
     plan = ctx.plan(rf(), grid, capi.bf_config(f_number=1.0))
     assert plan.variant() == 0
     plan.close()
+
+
+def test_tuning_that_fails_leaves_the_plan_as_it_was(gpu):
+    """A learned plan without its network cannot be tuned: it keeps the rule's
+    shape, and a shape that was set stays set."""
+    torch, capi, ctx = gpu
+    _, channel = probe_channel(capi, 3)
+    grid = capi.Grid(0, *image_points())
+    d = torch.zeros((3, 40, 260), dtype=torch.complex64, device="cuda")
+    out = torch.zeros(grid.shape, dtype=torch.complex64, device="cuda")
+    plan = ctx.plan(channel(), grid, capi.bf_config(f_number=1.0, combiner=3))
+    before = plan.variant()
+    assert before != 0
+    for v in (before, 6):
+        with pytest.raises(Exception, match="no network"):
+            plan.autotune(d.data_ptr(), out.data_ptr(), 1)
+        assert plan.variant() == v
+        plan.set_variant(6)
+    plan.close()

@@ -2655,6 +2655,9 @@ int usx_cu_bf_plan_autotune(usx_bf_plan* plan, const void* data, float* frame, i
   USX_CUDA(cudaEventCreate(&e0));
   USX_CUDA(cudaEventCreate(&e1));
   int best = plan->das_variant;
+  // A run that fails leaves the plan as it was.
+  const int saved_variant = plan->das_variant;
+  const bool saved_set = plan->variant_set;
   plan->variant_set = true;
   float best_ms = 0.0f;
   int rc = USX_OK;
@@ -2683,7 +2686,8 @@ int usx_cu_bf_plan_autotune(usx_bf_plan* plan, const void* data, float* frame, i
   ctx->profiling = saved_prof;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  plan->das_variant = best;
+  plan->das_variant = rc == USX_OK ? best : saved_variant;
+  plan->variant_set = rc == USX_OK || saved_set;
   if (rc != USX_OK) return rc;
   // Leave the caller's frame holding the chosen variant's result (all
   // variants agree bit for bit, so this is the same frame).
