@@ -241,3 +241,18 @@ def test_tuning_that_fails_leaves_the_plan_as_it_was(gpu):
         assert plan.variant() == v
         plan.set_variant(6)
     plan.close()
+
+
+@pytest.mark.parametrize("n_el,n0,n1,n_ev,cfg,kind", [
+    (2, 512, 1024, 1, {}, 0), (4, 512, 1024, 75, {}, 0), (8, 512, 1024, 1, {}, 0), (6, 512, 1024, 11, dict(compounding=2), 0),
+    (32, 1, 200000, 11, {}, 0), (64, 2, 100000, 40, {}, 0),
+    (8, 512, 1024, 20, {}, 4), (2, 16, 40, 3, {}, 4), (9, 512, 1024, 1, {}, 4), (128, 1, 200000, 11, {}, 4)])
+def test_the_shape_of_few_channels_and_thin_grids(gpu, n_el, n0, n1, n_ev, cfg, kind):
+    """Where channel warps or tiles would stay empty, a thread per pixel."""
+    torch, capi, ctx = gpu
+    _, channel = probe_channel(capi, n_ev, n_el=n_el)
+    ax0, ax1 = np.linspace(-5e-3, 5e-3, n0).astype(np.float32), np.linspace(1e-3, 9e-3, n1).astype(np.float32)
+    pts = np.stack(np.broadcast_arrays(ax0[:, None], 0.0, ax1[None]), -1).astype(np.float32)
+    plan = ctx.plan(channel(), capi.Grid(0, ax0, ax1, pts.reshape(-1, 3)), capi.bf_config(f_number=1.0, **cfg))
+    assert capi.das_variants()[plan.variant()][5] == kind
+    plan.close()

@@ -1841,16 +1841,45 @@ bool finite_transmit(const TxDev& t) {
 //     pixels, 61 against 74 (2) and 86 (22); 128 x 512, 105 / 99 / 95;
 //   more than 56 events: the table of a larger tile leaves too few CTAs per SM
 //     (256 x 512 pixels, 56 events: 570 (1), 548 (2), 559 (22); 64 events:
-//     638, 718, 1024);
+//     638, 718, 1024); select tables one event;
 //   up to 16 events: 128-pixel tiles (22) share the traces best (3 events:
-//     145 (1), 123 (2), 111 (22); 24 events: 296, 269, 271);
-//   else 64-pixel tiles (2).
-int default_variant(int n0, int n1, int n_frames, int events, int sm_count) {
+//     145 (1), 123 (2), 111 (22); 24 events: 296, 269, 271), but four lines x
+//     32 depths are mostly empty below 24 depths (30,000 x 3 pixels, 11 events:
+//     991, and 332 (2));
+//   else 64-pixel tiles (2), whose eight lines are half empty below five lines
+//     (3 x 100,000, 40 events: 2,195, and 1,473 (22)).
+// The thread-per-pixel kernel (0) stays the better one
+//   for one or two lines of many depths, whose tiles are half empty at best: 32
+//     channels, 1 x 200,000 pixels, 11 events, 312 (22) and 267 (0); 64
+//     channels, 2 x 100,000, 75 events, 1,297 (1) and 1,077 (0);
+//   for a probe of up to eight channels, which leave most of the 8 to 32
+//     channel warps idle: 4 channels, 512 x 1024 pixels, one event 77 (22) and
+//     38 (0), 11 events 133 and 106; 8 channels, 80 and 62, 11 events 141 and
+//     165. Its time and the tiles', in us, follow the two sums below within 15%
+//     over 1 to 8 channels, 1 to 150 events and 16 Ki to 512 Ki pixels.
+int default_variant(int n0, int n1, int n_frames, int events, int n_ch, bool select, int sm_count) {
   const long tiles = static_cast<long>(ceil_div(n0, 4)) * ceil_div(n1, 8) * n_frames;
   const long pixels = static_cast<long>(n0) * n1 * n_frames;
-  if (tiles <= sm_count) return 3;
-  if (pixels <= 48 * 1024 || events > 56) return 1;
-  return events <= 16 ? 22 : 2;
+  const int summed = select ? 1 : events;   // events a pixel sums
+  int v;
+  if (tiles <= sm_count)
+    v = 3;
+  else if (pixels <= 48 * 1024 || summed > 56)
+    v = 1;
+  else if (n0 <= 4)
+    v = 22;
+  else
+    v = n1 >= 24 && summed <= 16 ? 22 : 2;
+  if (n_ch > 8) return n0 <= 2 && pixels > 64 * 1024 && (n_ch <= 32 || summed > 16) ? 0 : v;
+  const int tl = v == 2 ? 8 : 4, td = v == 22 ? 32 : 8;   // the tile
+  const double c = n_ch, e = summed, others = events - summed, mega = n_frames / 524288.0;
+  const double p0 = mega * n0 * (32.0 * ceil_div(n1, 32));   // a warp of shape 0: one line, 32 depths
+  const double pv = mega * (static_cast<double>(tl) * ceil_div(n0, tl)) * (static_cast<double>(td) * ceil_div(n1, td));
+  const double t0 = 8.5 + 1.1 * c + 0.84 * e + 0.16 * c * e + 0.2 * others +
+                    p0 * (2.5 + 3.7 * c + 2.6 * e + 0.68 * c * e + 1.85 * others);
+  const double tv = v == 2 || v == 22 ? 8.8 + 0.2 * c + 0.23 * e + pv * (39.0 + 3.6 * c + 5.9 * e + 0.13 * c * e + 1.3 * others)
+                                      : 9.9 + 0.2 * c + 0.18 * e + pv * (46.0 + 6.1 * c + 9.2 * e + 0.18 * c * e + 1.3 * others);
+  return t0 < tv ? 0 : v;
 }
 
 // ------------------------------------------------------------------------
@@ -2193,7 +2222,8 @@ bool channel_warp_plan(const usx_bf_plan* p) { return channel_warp_samples(p->cd
 int plan_variant(const usx_bf_plan* p, int n_frames, int events) {
   if (p->variant_set || !p->cd.is_iq || p->cfg.compounding == USX_COMP_INCOHERENT || !channel_warp_plan(p) || events <= 0)
     return p->das_variant;
-  return default_variant(p->n0, p->n1, n_frames, events, p->ctx->sm_count);
+  return default_variant(p->n0, p->n1, n_frames, events, p->cd.probe.n_elements, p->cfg.compounding == USX_COMP_SELECT,
+                         p->ctx->sm_count);
 }
 
 int bf_execute(usx_bf_plan* plan, int n_frames, const void* data, int64_t data_stride,
