@@ -689,26 +689,32 @@ bool flow_lines_pay(const FlowArgs& a, int max_n, int count, size_t smem) {
   return (a.kl == 1 || a.kl == 2) && max_n >= 8 && pixels >= (a.kl == 1 ? 120000 : 40000) && smem <= 200 * 1024 &&
          ceil_div(a.n0, kFlowLines) <= 65535;
 }
+// ctx: for the profiler, which gets the name of the kernel that runs (null: none).
 template <typename Args, typename Pixel, typename Lines>
-int launch_flow_sums(cudaStream_t st, const FlowArgs& a, const Args& args, int max_n, int count, Pixel pixel,
-                     Lines lines1, Lines lines2) {
+int launch_flow_sums(usx_ctx* ctx, cudaStream_t st, const FlowArgs& a, const Args& args, int max_n, int count,
+                     Pixel pixel, Lines lines1, Lines lines2, const char* pixel_name, const char* lines_name) {
   const size_t smem = sizeof(float2) * static_cast<size_t>(max_n) * (kFlowCols + 2 * static_cast<size_t>(a.ka) + 1);
-  if (!flow_lines_pay(a, max_n, count, smem)) {
-    pixel<<<dim3(ceil_div(static_cast<long>(a.n0) * a.n1, 128), count), 128, 0, st>>>(args);
-    return USX_OK;
-  }
+  const bool lines = flow_lines_pay(a, max_n, count, smem);
+  const char* name = lines ? lines_name : pixel_name;
   Lines kern = a.kl == 1 ? lines1 : lines2;
-  if (smem > 48 * 1024)
+  if (lines && smem > 48 * 1024)
     if (int rc_ = smem_limit(reinterpret_cast<const void*>(kern), smem)) return rc_;
-  kern<<<dim3(ceil_div(a.n1, kFlowCols), ceil_div(a.n0, kFlowLines), count), kFlowCols, smem, st>>>(args);
+  if (ctx) prof_begin(ctx, name);
+  if (lines)
+    kern<<<dim3(ceil_div(a.n1, kFlowCols), ceil_div(a.n0, kFlowLines), count), kFlowCols, smem, st>>>(args);
+  else
+    pixel<<<dim3(ceil_div(static_cast<long>(a.n0) * a.n1, 128), count), 128, 0, st>>>(args);
+  if (ctx) prof_end(ctx);
+  USX_CHECK_LAUNCH(name);
   return USX_OK;
 }
-int launch_flow_sums(cudaStream_t st, const FlowArgs& a) {
-  return launch_flow_sums(st, a, a, a.n, 1, flow_kernel, flow_lines_kernel<1>, flow_lines_kernel<2>);
+int launch_flow_sums(usx_ctx* ctx, cudaStream_t st, const FlowArgs& a) {
+  return launch_flow_sums(ctx, st, a, a, a.n, 1, flow_kernel, flow_lines_kernel<1>, flow_lines_kernel<2>, "flow_kernel",
+                          "flow_lines_kernel");
 }
-int launch_flow_sums(cudaStream_t st, const FlowBatchArgs& b, int max_n, int count) {
-  return launch_flow_sums(st, b.base, b, max_n, count, flow_batch_kernel, flow_lines_batch_kernel<1>,
-                          flow_lines_batch_kernel<2>);
+int launch_flow_sums(usx_ctx* ctx, const FlowBatchArgs& b, int max_n, int count) {
+  return launch_flow_sums(ctx, ctx->stream, b.base, b, max_n, count, flow_batch_kernel, flow_lines_batch_kernel<1>,
+                          flow_lines_batch_kernel<2>, "flow_batch_kernel", "flow_lines_batch_kernel");
 }
 
 int launch_flow(usx_ctx* ctx, const float* filt, int n, int n0, int n1, float dz, float fdem,
@@ -734,10 +740,7 @@ int launch_flow(usx_ctx* ctx, const float* filt, int n, int n0, int n1, float dz
   a.pmax_bits = pmax_bits;
   const long n_pix = static_cast<long>(n0) * n1;
   USX_CUDA(cudaMemsetAsync(pmax_bits, 0, sizeof(unsigned), ctx->stream));
-  prof_begin(ctx, "flow_kernel");
-  if (int rc = launch_flow_sums(ctx->stream, a)) return rc;
-  prof_end(ctx);
-  USX_CHECK_LAUNCH("flow_kernel");
+  if (int rc = launch_flow_sums(ctx, ctx->stream, a)) return rc;
   const float ratio = std::pow(10.0f, cfg.power_threshold_db / 10.0f);
   prof_begin(ctx, "power_gate_kernel");
   power_gate_kernel<<<ceil_div(n_pix, 256), 256, 0, ctx->stream>>>(power, valid, n_pix, ratio, pmax_bits);
@@ -926,10 +929,7 @@ int usx_cu_color_flow_batch(usx_ctx* ctx, const float* ens, int n_ens, const int
     wall_batch_kernel<<<dim3(ceil_div(n_pix, threads), count), threads, smem, ctx->stream>>>(w);
     prof_end(ctx);
     USX_CHECK_LAUNCH("wall_batch_kernel");
-    prof_begin(ctx, "flow_batch_kernel");
-    if (int rc = launch_flow_sums(ctx->stream, fb, chunk_max, count)) return rc;
-    prof_end(ctx);
-    USX_CHECK_LAUNCH("flow_batch_kernel");
+    if (int rc = launch_flow_sums(ctx, fb, chunk_max, count)) return rc;
     e0 += count;
   }
   const float ratio = std::pow(10.0f, cfg->power_threshold_db / 10.0f);
@@ -999,8 +999,7 @@ int usx_cu_color_flow_noalloc(void* stream, const float* ens, int n_frames, int 
   f.pmax_bits = pmax_bits;
   // The scratch keeps the previous call's contents: the running maximum must start at zero.
   USX_CUDA(cudaMemsetAsync(pmax_bits, 0, sizeof(unsigned), st));
-  if (int rc = launch_flow_sums(st, f)) return rc;
-  USX_CHECK_LAUNCH("flow_kernel");
+  if (int rc = launch_flow_sums(nullptr, st, f)) return rc;
   const float ratio = std::pow(10.0f, cfg->power_threshold_db / 10.0f);
   power_gate_kernel<<<ceil_div(n_pix, 256), 256, 0, st>>>(power, valid, n_pix, ratio, pmax_bits);
   USX_CHECK_LAUNCH("power_gate_kernel");
@@ -1036,8 +1035,10 @@ int usx_cu_axial_displacement(usx_ctx* ctx, const float* before, const float* af
   const long reach = static_cast<long>(p.ka) + std::max(1, p.lag_max);
   q.col_lo = static_cast<int>(std::min<long>(reach, n1));
   q.col_hi = static_cast<int>(std::max<long>(q.col_lo, n1 - reach));
-  prof_begin(ctx, "displacement_kernel");
-  if (disp_lines_pay(p, n) && p.lag_max <= kDispMaxLag && q.col_hi > q.col_lo) {
+  const bool lines = disp_lines_pay(p, n) && p.lag_max <= kDispMaxLag && q.col_hi > q.col_lo;
+  const char* name = lines ? "displacement_lines_kernel" : "displacement_kernel";
+  prof_begin(ctx, name);
+  if (lines) {
     q.col_blocks = ceil_div(q.col_hi - q.col_lo, kDispCols);
     q.n_edge = ceil_div(static_cast<long>(n0) * (n1 - (q.col_hi - q.col_lo)), kDispCols);
     const unsigned grid = static_cast<unsigned>(q.n_edge + static_cast<long>(q.col_blocks) * ceil_div(n0, kDispLines));
@@ -1048,7 +1049,7 @@ int usx_cu_axial_displacement(usx_ctx* ctx, const float* before, const float* af
     displacement_kernel<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(p);
   }
   prof_end(ctx);
-  USX_CHECK_LAUNCH("displacement_kernel");
+  USX_CHECK_LAUNCH(name);
   return USX_OK;
 }
 
