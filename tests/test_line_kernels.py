@@ -73,3 +73,62 @@ def test_the_profiler_names_the_kernel_that_ran(gpu):
         ens.data_ptr(), [16, 8], [0, 16], 256, 512, axis(512), 5e6, 5e3, 1540.0, capi.doppler_config(),
         *[m.data_ptr() for m in maps]))
     assert "flow_lines_batch_kernel" in got and "flow_batch_kernel" not in got
+
+
+@pytest.mark.parametrize("n,n0,n1,ka,kl,lines", [
+    (16, 256, 512, 4, 1, True), (12, 200, 512, 6, 2, True), (8, 500, 1000, 1, 1, True), (32, 60, 700, 4, 2, True),
+    (32, 3000, 40, 4, 1, False), (16, 1000, 130, 4, 1, False),    # blocks mostly empty in depth
+    (32, 256, 512, 0, 1, False), (32, 256, 512, 1, 1, False),     # windows that do not pay for the staging
+    (32, 400, 128, 6, 2, True), (12, 400, 128, 6, 2, False),      # one block in depth
+    (12, 60, 700, 2, 2, False), (16, 1, 150000, 4, 2, False),     # too few blocks, no second line
+    (5, 500, 1000, 4, 1, False), (16, 256, 512, 4, 3, False)])
+def test_colour_flow_kernel_by_size(gpu, n, n0, n1, ka, kl, lines):
+    torch, capi, ctx = gpu
+    assert ("flow_lines_kernel" in flow_kernels(capi, torch, ctx, n, n0, n1, ka, kl)) == lines
+
+
+@pytest.mark.parametrize("n,n0,n1,ka,kl", [(8, 261, 640, 4, 1), (33, 183, 500, 6, 2), (9, 500, 999, 1, 2),
+                                           (64, 255, 512, 3, 1)])
+def test_colour_flow_lines_equal_a_pixel_per_thread(gpu, n, n0, n1, ka, kl):
+    """A hundred columns of the same ensemble run a pixel per thread; away from
+    their cut edges every sum is over the same terms in the same order. (The
+    valid bytes pass the power gate, which depends on the frame's maximum.)"""
+    torch, capi, ctx = gpu
+    ens = speckle(torch, (n, n0, n1), n)
+    ens[:, 7, 300:340] = 0
+    ens[1, 20, 330] = float("nan")
+    ens[2, 40, 310] = float("inf")
+    cfg = dict(kernel_axial=ka, kernel_lateral=kl, power_threshold_db=-300.0, coherence_threshold=0.05, polynomial_order=0)
+    whole, part = flow_maps(torch, (n0, n1)), flow_maps(torch, (n0, 100))
+    assert "flow_lines_kernel" in kernels(capi, torch, ctx, lambda: flow(ctx, capi, ens, whole, **cfg))
+    for j0 in (0, 128 - 50, 300, n1 - 100):
+        cut = ens[:, :, j0:j0 + 100].contiguous()
+        assert "flow_kernel" in kernels(capi, torch, ctx, lambda: flow(ctx, capi, cut, part, **cfg))
+        lo, hi = (0 if j0 == 0 else ka + 1), (100 if j0 == n1 - 100 else 100 - ka - 1)
+        for w, p in zip(whole[:3], part):
+            w, p = w[:, j0 + lo:j0 + hi].cpu().numpy(), p[:, lo:hi].cpu().numpy()
+            assert np.array_equal(w, p, equal_nan=True)
+    assert (whole[0] != 0).sum() > 1000   # coherent pixels have a velocity
+
+
+@pytest.mark.parametrize("ka,kl", [(4, 1), (3, 2)])
+def test_uneven_batches_equal_one_ensemble_at_a_time(gpu, ka, kl):
+    """Ensembles of 32, 2, 7 and 9 frames in one four-line launch; alone, those
+    below eight frames run a pixel per thread."""
+    torch, capi, ctx = gpu
+    frames, n0, n1 = [32, 2, 7, 9], 256, 512
+    ens = speckle(torch, (sum(frames), n0, n1), 3)
+    cfg = dict(kernel_axial=ka, kernel_lateral=kl, coherence_threshold=0.05, polynomial_order=0)
+    off = [0, 32, 34, 41]
+    maps = flow_maps(torch, (4, n0, n1))
+    got = kernels(capi, torch, ctx, lambda: ctx.color_flow_batch(
+        ens.data_ptr(), frames, off, n0, n1, axis(n1), 5e6, 5e3, 1540.0, capi.doppler_config(**cfg),
+        *[m.data_ptr() for m in maps]))
+    assert "flow_lines_batch_kernel" in got
+    for e, (n, o) in enumerate(zip(frames, off)):
+        one = flow_maps(torch, (n0, n1))
+        names = kernels(capi, torch, ctx, lambda: flow(ctx, capi, ens[o:o + n].contiguous(), one, **cfg))
+        assert ("flow_kernel" in names) == (n < 8)
+        for m, w in zip(maps, one):
+            assert torch.equal(m[e], w)
+        assert (one[3] == 1).any()

@@ -677,17 +677,30 @@ int launch_wall(usx_ctx* ctx, const float* ens, int n, long n_pix, int type, int
   return USX_OK;
 }
 
-// The flow sums of `count` ensembles of at most max_n frames. Four lines per
-// thread where the windows span lines (kl of 1 or 2) and a quarter of the
-// pixels as threads still fills the GPU (wall filter and gate included, us,
-// pixel per thread against four lines; 9 x 3 windows: one ensemble of 32
-// frames, 64 x 256, 65 / 98; 256 x 512, 165 / 143; 8 frames, 50 / 45; two of
-// 4 and 6 frames, 256 x 256, 41 / 51; 13 x 5 windows, 24 frames, 256 x 256:
-// 154 / 116; 9 x 5, 32 frames, 121 x 333: 139 / 119; 5 x 1: 232 / 269).
+// The flow sums of `count` ensembles of at most max_n frames: four lines per
+// thread where the windows span lines (kl of 1 or 2) and the blocks are full of
+// work: kFlowCols depths each, so that the depths must fill most of them (fill;
+// 130 of 256: 1.0 to 1.6 times the time of a pixel per thread at 9 depths a
+// window; 200 of 256: equal), enough of them for the SMs, and enough window terms to
+// pay for the staging, which a short window does not. Time with four lines over
+// that with a pixel per thread (this kernel alone):
+//   kl = 1: 256 x 512, 8 to 64 frames, 3 depths a window 1.07 to 1.37, 7 depths
+//     0.87 to 1.05, 9 depths 0.79 to 0.96, 13 depths 0.74 to 0.88; 180 x 380 (135
+//     blocks), 13 depths 0.76 to 1.22; 640 x 200, 9 depths 1.00 to 1.12;
+//   kl = 2: 256 x 512, 5 depths 0.73 to 0.96; 60 x 700 (90 blocks), 9 depths, 8 /
+//     32 / 64 frames 1.07 / 0.84 / 0.67; 128 x 330, 32 frames, 9 depths 0.83;
+//     400 x 128 (one block in depth), 24 / 32 / 64 frames 1.06 / 0.96 / 0.68.
+// Of 3,984 such shapes, 3 to 25 depths, the rule takes a thousand, sixteen of them
+// at a loss of more than 3% (at most 1.19).
 bool flow_lines_pay(const FlowArgs& a, int max_n, int count, size_t smem) {
-  const long pixels = static_cast<long>(a.n0) * a.n1 * count;
-  return (a.kl == 1 || a.kl == 2) && max_n >= 8 && pixels >= (a.kl == 1 ? 120000 : 40000) && smem <= 200 * 1024 &&
-         ceil_div(a.n0, kFlowLines) <= 65535;
+  if ((a.kl != 1 && a.kl != 2) || a.ka < 1 || max_n < 8 || a.n0 < 2 || smem > 200 * 1024 ||
+      ceil_div(a.n0, kFlowLines) > 65535 || (a.n1 <= kFlowCols && (a.kl == 1 || max_n < 32)))
+    return false;
+  const double cols = ceil_div(a.n1, kFlowCols), fill = a.n1 / (cols * kFlowCols);
+  const double blocks = cols * ceil_div(a.n0, kFlowLines) * count;
+  const double work = static_cast<double>(a.n0) * a.n1 * count * fill * fill * (2.0 * a.ka + 1);
+  return fill >= 0.65 &&
+         (a.kl == 1 ? blocks >= 152 && work >= 9e5 : blocks >= 88 && work * std::sqrt(max_n / 16.0) >= 4e5);
 }
 // ctx: for the profiler, which gets the name of the kernel that runs (null: none).
 template <typename Args, typename Pixel, typename Lines>
