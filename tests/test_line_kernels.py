@@ -132,3 +132,39 @@ def test_uneven_batches_equal_one_ensemble_at_a_time(gpu, ka, kl):
         for m, w in zip(maps, one):
             assert torch.equal(m[e], w)
         assert (one[3] == 1).any()
+
+
+@pytest.mark.parametrize("n0,n1,ka,kl,lag,lines", [
+    (256, 1024, 8, 2, 8, True), (256, 300, 4, 2, 4, True), (128, 512, 12, 0, 8, True), (2000, 80, 4, 2, 8, True),
+    (20000, 12, 1, 2, 2, False), (5000, 30, 4, 1, 4, False), (2000, 50, 2, 0, 12, False),   # few interior columns
+    (128, 512, 1, 0, 30, False), (64, 256, 4, 0, 4, False), (1, 100000, 2, 2, 12, False), (1, 100000, 8, 2, 8, True),
+    (12, 64, 8, 2, 8, False),
+    (256, 1024, 4, 3, 8, False)])
+def test_displacement_kernel_by_size(gpu, n0, n1, ka, kl, lag, lines):
+    torch, capi, ctx = gpu
+    assert ("displacement_lines_kernel" in disp_kernels(capi, torch, ctx, n0, n1, ka, kl, lag)) == lines
+
+
+@pytest.mark.parametrize("n0,n1,ka,kl,lag", [(130, 700, 8, 2, 8), (257, 640, 3, 1, 5), (515, 400, 6, 0, 12)])
+def test_displacement_lines_equal_a_pixel_per_thread(gpu, n0, n1, ka, kl, lag):
+    """Six lines of the same frames run a pixel per thread; away from their cut
+    edges every sum is over the same terms in the same order."""
+    torch, capi, ctx = gpu
+    a = speckle(torch, (n0, n1), n0)
+    b = torch.roll(a, 3, 1) * np.exp(-0.4j) + 0.05 * speckle(torch, (n0, n1), 1)
+    a[7, 300:340] = 0
+    b[9, 200] = float("nan")
+    ax, cr = torch.full((n0, n1), 7.0, device="cuda"), torch.full((n0, n1), 7.0, device="cuda")
+
+    def run(x, y, m, c):
+        return kernels(capi, torch, ctx, lambda: ctx.axial_displacement(
+            x.data_ptr(), y.data_ptr(), x.shape[0], n1, axis(n1), 5e6, 1540.0, ka, kl, lag, m.data_ptr(), c.data_ptr()))
+
+    assert "displacement_lines_kernel" in run(a, b, ax, cr)
+    for i0 in (0, 61, n0 - 6):
+        m, c = torch.empty((6, n1), device="cuda"), torch.empty((6, n1), device="cuda")
+        assert "displacement_kernel" in run(a[i0:i0 + 6].contiguous(), b[i0:i0 + 6].contiguous(), m, c)
+        lo, hi = (0 if i0 == 0 else kl), (6 if i0 == n0 - 6 else 6 - kl)
+        for w, part in ((ax, m), (cr, c)):
+            assert np.array_equal(w[i0 + lo:i0 + hi].cpu().numpy(), part[lo:hi].cpu().numpy(), equal_nan=True)
+    assert (cr > 0).float().mean() > 0.5

@@ -636,14 +636,29 @@ __global__ void strain_kernel(const float* axial, int n0, int n1, float dz, int 
   strain[k] = out;
 }
 
-// Whether the four-line kernel pays (window terms x lags per pixel; us, a pixel
-// per thread against four lines): 64 x 256 pixels, 225 terms 33 / 41, 243
-// terms 35 / 33; 256 x 512, 9 terms 19 / 23, 63 terms 29 / 29, 243 terms 65 /
-// 41; 256 x 1024, 1,445 terms 513 / 169; 12 x 64, 1,445 terms 131 / 125: few
-// terms over few pixels only pay for the block's set-up.
-bool disp_lines_pay(const DispArgs& p, long n_pix) {
-  const double terms = (2.0 * p.ka + 1) * (2.0 * p.kl + 1) * (2.0 * p.lag_max + 1);
-  return p.kl <= 2 && (terms >= 1000.0 || terms * static_cast<double>(n_pix) >= 8.4e6);
+// Whether the four-line kernel pays over the `interior` columns of n0 lines. Its
+// blocks are kDispCols columns x kDispLines lines and form kDispLags lags at a
+// time, so what counts is the window terms x lags (terms) over the interior
+// pixels, times the shares of the blocks' columns and lines and of the lags that
+// are wanted; from two blocks per SM on, less of it. (Time with four lines over
+// that with a pixel per thread, this kernel alone: 256 x 1024, 85 terms x 17 lags
+// 0.31; 256 x 300, 45 x 9 0.46; 64 x 256, 27 x 9 0.93; 20,000 x 12, 15 x 5, eight
+// interior columns 2.9; 5,000 x 30, 9 x 17 1.7; 2,000 x 50, 5 x 25 1.5.) Without
+// lines to share (kl = 0, or a single line) a lag of a short window costs its
+// set-up: 128 x 512, 3 x 61 1.5, 9 x 25 1.07, 17 x 17 0.8; 256 x 1024, 5 x 17 0.73;
+// 1 x 100,000, 5 x 25 1.24, 17 x 17 0.70. Of 3,105 such shapes the rule takes
+// 948, fourteen of them at a loss of more than 3% (at most 1.10).
+bool disp_lines_pay(const DispArgs& p, int interior) {
+  if (p.kl > 2 || p.lag_max > kDispMaxLag || interior <= 0) return false;
+  const int kl = p.n0 == 1 ? 0 : p.kl;
+  const double blocks = static_cast<double>(ceil_div(p.n0, kDispLines)) * ceil_div(interior, kDispCols);
+  const bool many = blocks >= 300;
+  if (kl == 0 && ((p.ka < 4 && (!many || p.n0 == 1)) || (p.n0 == 1 && p.lag_max < 4))) return false;
+  const double fill = interior / (static_cast<double>(kDispCols) * ceil_div(interior, kDispCols));
+  const double lines = p.n0 == 1 ? 1.0 : p.n0 * static_cast<double>(p.n0) / (kDispLines * ceil_div(p.n0, kDispLines));
+  const double lags = 2.0 * p.lag_max + 1, passes = kDispLags * std::ceil(lags / kDispLags);
+  const double terms = (2.0 * p.ka + 1) * (2.0 * kl + 1) * lags * (lags / passes);
+  return fill >= 0.25 && terms * lines * interior * fill >= (kl == 0 ? 1e7 : many ? 3e6 : 5e6);
 }
 
 float axial_step(const float* axis1, int n1) {
@@ -1048,7 +1063,7 @@ int usx_cu_axial_displacement(usx_ctx* ctx, const float* before, const float* af
   const long reach = static_cast<long>(p.ka) + std::max(1, p.lag_max);
   q.col_lo = static_cast<int>(std::min<long>(reach, n1));
   q.col_hi = static_cast<int>(std::max<long>(q.col_lo, n1 - reach));
-  const bool lines = disp_lines_pay(p, n) && p.lag_max <= kDispMaxLag && q.col_hi > q.col_lo;
+  const bool lines = disp_lines_pay(p, q.col_hi - q.col_lo);
   const char* name = lines ? "displacement_lines_kernel" : "displacement_kernel";
   prof_begin(ctx, name);
   if (lines) {
