@@ -256,3 +256,14 @@ def test_the_shape_of_few_channels_and_thin_grids(gpu, n_el, n0, n1, n_ev, cfg, 
     plan = ctx.plan(channel(), capi.Grid(0, ax0, ax1, pts.reshape(-1, 3)), capi.bf_config(f_number=1.0, **cfg))
     assert capi.das_variants()[plan.variant()][5] == kind
     plan.close()
+
+
+@pytest.mark.parametrize("n,wall", [(5, 0), (12, 1), (33, 2), (9, 2)])
+def test_wall_filter_in_place(gpu, n, wall):
+    torch, capi, ctx = gpu
+    rng = np.random.default_rng(n)
+    z = torch.from_numpy((rng.normal(size=(n, 1000)) + 1j * rng.normal(size=(n, 1000))).astype(np.complex64)).cuda()
+    out = torch.empty_like(z)
+    ctx.wall_filter(z.data_ptr(), n, 1000, wall, 2, out.data_ptr())
+    ctx.wall_filter(z.data_ptr(), n, 1000, wall, 2, z.data_ptr())
+    assert torch.equal(z, out)

@@ -63,59 +63,60 @@ struct WallArgs {
   float M[kMaxEns * kMaxEns];
 };
 
-// The wall filter's shared memory: the block's ensembles z[n][kWallThreads],
-// then the projector transposed, Mt[j][i] with rows of kWallRows multiples.
+// The wall filter: a pixel per thread, its ensemble z[n][kWallThreads] in shared
+// memory, filtered frame i of src[j * n_pix] through the n x n projector M to
+// store(i, value), ascending i. Eight rows at a time share each read of z; M is
+// read where the kernel's arguments lie; every row sums over j in ascending
+// order, products and sums rounded separately. (in: the pixel exists. src may be
+// the frames that store writes: a thread reads its pixel whole before it writes,
+// and by ordinary loads.)
+// What bounds it: latency at the occupancy that 1 KB per frame and block leaves.
+// Polynomial filter of order 2, 131,072 pixels, us, a row at a time / eight: 8
+// frames 10.4 / 10.5, 16 18.8 / 16.2, 32 43 / 42, 48 95 / 80, 64 181 / 143. With M
+// transposed in shared memory as well, for 16-byte reads of it: 17.5, 43, 140 and
+// 222 from 16 frames on (fewer blocks beside one another); 524,288 pixels, 16
+// frames, 39.6 against 47.4 here.
 constexpr int kWallThreads = 128, kWallRows = 8;
-__host__ __device__ constexpr int wall_pitch(int n) { return (n + kWallRows - 1) / kWallRows * kWallRows; }
-__host__ __device__ constexpr size_t wall_smem(int n) {
-  return sizeof(float2) * n * kWallThreads + sizeof(float) * n * wall_pitch(n);
-}
+__host__ __device__ constexpr size_t wall_smem(int n) { return sizeof(float2) * n * kWallThreads; }
 
-// One pixel's ensemble src[j * n_pix] through the n x n projector M: filtered
-// frame i goes to store(i, value), ascending i. Eight rows at a time share each
-// read of z and two 16-byte reads of Mt; every row sums over j in ascending
-// order, products and sums rounded separately. Every thread of the block calls
-// it (in: the pixel exists).
 template <typename Store>
 __device__ __forceinline__ void wall_pixel(float4* smem, const float2* src, long n_pix, int n, const float* M,
                                            bool identity, bool in, Store store) {
+  if (!in) return;
   float2* z = reinterpret_cast<float2*>(smem) + threadIdx.x;
-  float* Mt = reinterpret_cast<float*>(reinterpret_cast<float2*>(smem) + n * kWallThreads);
-  const int pitch = wall_pitch(n);
-  if (in)
 #pragma unroll 8
-    for (int j = 0; j < n; ++j) z[j * kWallThreads] = __ldg(src + j * n_pix);
+  for (int j = 0; j < n; ++j) z[j * kWallThreads] = src[j * n_pix];
   if (identity) {
-    if (in)
-      for (int i = 0; i < n; ++i) store(i, z[i * kWallThreads]);
+    for (int i = 0; i < n; ++i) store(i, z[i * kWallThreads]);
     return;
   }
-  for (int q = threadIdx.x; q < n * pitch; q += kWallThreads) {
-    const int j = q / pitch, i = q - j * pitch;
-    Mt[q] = i < n ? M[i * n + j] : 0.0f;
-  }
-  __syncthreads();
-  if (!in) return;
-  for (int i = 0; i < n; i += kWallRows) {
+  int i = 0;
+  for (; i + kWallRows <= n; i += kWallRows) {
     float2 acc[kWallRows];
 #pragma unroll
     for (int r = 0; r < kWallRows; ++r) acc[r] = make_float2(0.f, 0.f);
 #pragma unroll 2
     for (int j = 0; j < n; ++j) {
       const float2 v = z[j * kWallThreads];
-      float m[kWallRows];
-      const float4* row = reinterpret_cast<const float4*>(Mt + j * pitch + i);
-      *reinterpret_cast<float4*>(m) = row[0];
-      *reinterpret_cast<float4*>(m + 4) = row[1];
 #pragma unroll
       for (int r = 0; r < kWallRows; ++r) {
-        acc[r].x += v.x * m[r];
-        acc[r].y += v.y * m[r];
+        const float m = M[(i + r) * n + j];
+        acc[r].x += v.x * m;
+        acc[r].y += v.y * m;
       }
     }
 #pragma unroll
-    for (int r = 0; r < kWallRows; ++r)
-      if (i + r < n) store(i + r, acc[r]);
+    for (int r = 0; r < kWallRows; ++r) store(i + r, acc[r]);
+  }
+  for (; i < n; ++i) {
+    float2 acc = make_float2(0.f, 0.f);
+    for (int j = 0; j < n; ++j) {
+      const float2 v = z[j * kWallThreads];
+      const float m = M[i * n + j];
+      acc.x += v.x * m;
+      acc.y += v.y * m;
+    }
+    store(i, acc);
   }
 }
 
