@@ -273,10 +273,12 @@ __global__ void init_uniform_kernel(float* p, long n, float a, unsigned long lon
 }
 
 // dY = 2 (Y - T) * mask / count over the valid outputs; loss sum into *loss.
-// Bound by the loss's atomics, one per warp onto one word (26.7 us at 4,096 x 128).
-// Block sums take 5.7 us, but round the total another way: 5 of 60 batches then
-// lie 1.5 times further from the 64-bit loss (its BF16 error of 1e-6 to 2e-5
-// included), 1 of 60 from one run of this kernel to the next.
+// Bound by the loss's atomics, one per warp onto one word (26.7 us at 4,096 x
+// 128), which leave it within 3.4e-6 of the 64-bit sum of the same outputs. Block
+// sums take 5.7 us and come within 6e-7, but round the total another way: beside
+// the BF16 forward's own error of 1e-6 to 2e-5 that moves the loss away from the
+// 64-bit network's on some batches and towards it on others (more than 1.5 times
+// further on 5 of 60; on 1 from one run of this kernel to the next).
 __global__ void mse_grad_kernel(const float* y, const float* t, const float* mask, long rows, int n_out,
                                 int ld, float inv_count, float* dy32, __nv_bfloat16* dy16, float* loss) {
   const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;

@@ -73,7 +73,7 @@ constexpr int kMaxTimeTable = 8192;
 // Incident samples a warp keeps in shared memory; a longer window (up to the
 // clamp) uses the warp's slot of a global-memory buffer instead.
 constexpr int kIncSmall = 1536;
-constexpr int kTimeSlack = 128;   // sample times past the record (read, not used)
+constexpr int kTimeSlack = 32;   // sample times past the record (read, not used)
 
 struct SimArgs {
   const usx_scatterer* scat;
@@ -188,8 +188,9 @@ template <bool kTable>
 __global__ void __launch_bounds__(32 * kSimWarps) simulate_kernel(const SimArgs a) {
   extern __shared__ float4 sim_smem[];
   // Shared memory: per warp an element table and a small incident buffer, then
-  // the pulse and the sample-time table (read up to 127 past its end by lanes
-  // that store nothing; kTimeSlack words follow it).
+  // the pulse and the sample-time table. Lanes that store nothing read past an
+  // element's last sample n1: every step has its first lanes' samples within it
+  // (n + 96, n + 32 or n at most n1), so that the last lane reads n1 + 31 at most.
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float4* e_tab = sim_smem + warp * (a.inc_small / 4 + a.tbl_pad);   // [tbl_pad]
   float* inc_smem = reinterpret_cast<float*>(e_tab + a.tbl_pad);     // [inc_small]
