@@ -267,3 +267,26 @@ def test_wall_filter_in_place(gpu, n, wall):
     ctx.wall_filter(z.data_ptr(), n, 1000, wall, 2, out.data_ptr())
     ctx.wall_filter(z.data_ptr(), n, 1000, wall, 2, z.data_ptr())
     assert torch.equal(z, out)
+
+
+@pytest.mark.parametrize("n0,n1", [(1, 3), (2, 9), (7, 5), (16, 40)])
+def test_scan_extent_keeps_the_first_zero_s_sign(gpu, n0, n1):
+    """Extents of zero: as one pass over the points keeps the first of equal
+    values, whichever zeros follow it."""
+    torch, capi, ctx = gpu
+    rng = np.random.default_rng(n0)
+    img, px = torch.zeros((n0, n1), device="cuda"), torch.empty((4, 4), device="cuda")
+    for side in (1.0, -1.0):
+        pts = (side * rng.random((n0 * n1, 3))).astype(np.float32)
+        pts[rng.random(pts.shape) < 0.2] = 0.0
+        pts[rng.random(pts.shape) < 0.2] = -0.0
+        pts[n0 * n1 // 3] = 0.0
+        got = ctx.scan_convert(img.data_ptr(), capi.Grid(0, np.linspace(-1, 1, n0), np.linspace(0, 1, n1), pts), 4, 4,
+                               0.0, px.data_ptr())
+        want = []
+        for c in (0, 2):
+            lo, hi = np.float32(np.finfo(np.float32).max), np.float32(-np.finfo(np.float32).max)
+            for v in pts[:, c]:
+                lo, hi = (v if v < lo else lo), (v if hi < v else hi)
+            want += [lo, hi]
+        assert np.asarray(got, np.float32).tobytes() == np.asarray(want, np.float32).tobytes()

@@ -257,18 +257,30 @@ Extent points_extent(const float* p, long n) {
     e.z_min = std::min(e.z_min, p[3 * k + 2]);
     e.z_max = std::max(e.z_max, p[3 * k + 2]);
   }
-  auto first_zero = [&](float& v, int c) {
+  // Every lane kept its own first zero, and the tail's are looked at: the points
+  // are searched only where the signs of those differ.
+  auto first_zero = [&](float& v, int c, const vec4 (&lanes)[6]) {
     if (v != 0.0f) return;
+    bool plus = false, minus = false;
+    auto see = [&](float z) {
+      if (z == 0.0f) (std::signbit(z) ? minus : plus) = true;
+    };
+    for (int i = c; i < 24; i += 3) see(lanes[i / 4][i % 4]);
+    for (long i = n / 8 * 8; i < n; ++i) see(p[3 * i + c]);
+    if (plus != minus) {
+      v = minus ? -0.0f : 0.0f;
+      return;
+    }
     for (long i = 0; i < n; ++i)
       if (p[3 * i + c] == 0.0f) {
         v = p[3 * i + c];
         return;
       }
   };
-  first_zero(e.x_min, 0);
-  first_zero(e.x_max, 0);
-  first_zero(e.z_min, 2);
-  first_zero(e.z_max, 2);
+  first_zero(e.x_min, 0, lo);
+  first_zero(e.x_max, 0, hi);
+  first_zero(e.z_min, 2, lo);
+  first_zero(e.z_max, 2, hi);
   return e;
 }
 }  // namespace
