@@ -290,3 +290,27 @@ def test_scan_extent_keeps_the_first_zero_s_sign(gpu, n0, n1):
                 lo, hi = (v if v < lo else lo), (v if hi < v else hi)
             want += [lo, hi]
         assert np.asarray(got, np.float32).tobytes() == np.asarray(want, np.float32).tobytes()
+
+
+def test_queues_of_few_channels_and_thin_grids(gpu):
+    """Both tiles of the queue, by its entries' work: each frame as alone."""
+    torch, capi, ctx = gpu
+    rng = np.random.default_rng(12)
+
+    def entry(n_el, n_ev, n0, n1, **cfg):
+        _, channel = probe_channel(capi, n_ev, n_el=n_el)
+        iq = (rng.normal(size=(n_ev, n_el, 260)) + 1j * rng.normal(size=(n_ev, n_el, 260))).astype(np.complex64)
+        grid = capi.Grid(0, *image_points(n0, n1))
+        want = frames_of(capi, torch, ctx, channel(), grid, iq, (0,), **cfg)[0]
+        return ctx.plan(channel(), grid, capi.bf_config(f_number=1.0, **cfg)), torch.from_numpy(iq).cuda(), want
+
+    few = [entry(3, 40, 30, 70), entry(24, 2, 9, 33, compounding=2), entry(1, 1, 1, 1)]
+    thin = [entry(64, 3, 2, 700), entry(40, 35, 1, 900)]
+    full = [entry(128, 5, 40, 50), entry(128, 83, 17, 20, compounding=2)]
+    for queue in (few, thin, full, few + thin + full, full[:1] + few):
+        out = [torch.full(w.shape, 7.0, dtype=torch.complex64, device="cuda") for _, _, w in queue]
+        ctx.execute_queue([p for p, _, _ in queue], [d.data_ptr() for _, d, _ in queue], [o.data_ptr() for o in out])
+        for o, (_, _, w) in zip(out, queue):
+            assert np.array_equal(o.cpu().numpy(), w)
+    for p, _, _ in few + thin + full:
+        p.close()

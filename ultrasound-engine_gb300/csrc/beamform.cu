@@ -860,9 +860,9 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_queue_kernel(const 
   }
 }
 
-// The same queue over das_csum_kernel's body (IQ plans): CTAs of 2 pixel
-// warps x 8 channel warps on 8-line x 8-depth tiles.
-template <bool kSel>   // some entry compounds by selection
+// The same queue over das_csum_kernel's body (IQ plans): CTAs of kPW pixel warps
+// x kCQ channel warps on tiles of kTL lines.
+template <int kPW, int kCQ, int kTL, bool kSel>   // kSel: some entry compounds by selection
 __global__ void __launch_bounds__(512, 2) das_csum_queue_kernel(const DasQueueArgs q) {
   __shared__ int s_item;
   const int total = q.first[q.n];
@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(512, 2) das_csum_queue_kernel(const DasQueueAr
     while (e + 1 < q.n && item >= q.first[e + 1]) ++e;
     const int local = item - q.first[e];
     const int frame = local / q.tiles[e], tile = local - frame * q.tiles[e];
-    das_export_body<4, 2, 8, 4, 8, true, kSel>(q.args[e], tile, frame);
+    das_export_body<4, kPW, kCQ, 4, kTL, true, kSel>(q.args[e], tile, frame);
   }
 }
 
@@ -2214,6 +2214,27 @@ BfArgs make_args(const usx_bf_plan* p) {
 }
 
 
+// The queue's tile: 4 lines x 32 depths with 4 pixel and 4 channel warps (slim), or
+// 8 x 8 with 2 and 8. A launch has one for all its entries: that of the greater
+// part of their work. Slim where few channels leave the eight channel warps idle
+// (16 channels, 3 events, four frames of 256 x 640: 181 us against 287; 64
+// channels, 31 events: 1,306 and 1,453; 128 channels, 75 events, 128 x 256: 1,011
+// and 802) and where eight lines would be mostly empty (128 channels, 3 events,
+// two frames of 2 x 20,000: 196 and 411), unless its 32 depths would be (16
+// channels, 3 events, four frames of 3,000 x 3: 111 and 70). It tabulates 32 events
+// at a time, so that two CTAs fit an SM.
+bool queue_slim(usx_bf_plan* const* plans, int n) {
+  double work[2] = {0.0, 0.0};
+  for (int k = 0; k < n; ++k) {
+    const usx_bf_plan* p = plans[k];
+    const int n_ch = p->cd.probe.n_elements;
+    const double wide = 64.0 * ceil_div(p->n0, 8) * ceil_div(p->n1, 8), slim = 128.0 * ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
+    const bool s = (n_ch <= 24 && slim <= 1.3 * wide) || wide > 1.5 * slim;
+    work[s] += static_cast<double>(p->n0) * p->n1 * n_ch * std::max(1, p->ev_end - p->ev_begin);
+  }
+  return work[1] > work[0];
+}
+
 // Whether the channel-warp kernels take the plan's traces and delays.
 bool channel_warp_plan(const usx_bf_plan* p) { return channel_warp_samples(p->cd.acq.n_samples) && p->finite_delays; }
 
@@ -2850,6 +2871,8 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     // Plans the channel-warp body does not take go to das_fast_kernel's tiles.
     bool cw = iq, any_select = false;
     for (int k = 0; k < m; ++k) cw = cw && channel_warp_plan(plans[i0 + k]);
+    const bool slim = queue_slim(plans + i0, m);
+    const int tl = slim ? 4 : 8, td = slim ? 32 : 8, cq = slim ? 4 : 8, pw = slim ? 4 : 2, most = slim ? 32 : kTabEvents;
     for (int k = 0; k < m; ++k) {
       const usx_bf_plan* p = plans[i0 + k];
       BfArgs a = make_args(p);
@@ -2864,11 +2887,10 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
         USX_CUDA(cudaMemsetAsync(frames[i0 + k], 0, sizeof(float2) * a.n_pix, ctx->stream));
         continue;
       }
-      const int tiles = cw ? ceil_div(p->n0, 8) * ceil_div(p->n1, 8) : ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
+      const int tiles = cw ? ceil_div(p->n0, tl) * ceil_div(p->n1, td) : ceil_div(p->n0, 4) * ceil_div(p->n1, 32);
       q.args[q.n] = a;
       any_select = any_select || a.compounding == USX_COMP_SELECT;
-      tab_events = std::max(tab_events, a.compounding == USX_COMP_SELECT ? 8   // (its channel warps)
-                                                                         : std::min(kTabEvents, a.ev_end - a.ev_begin));
+      tab_events = std::max(tab_events, a.compounding == USX_COMP_SELECT ? cq : std::min(most, a.ev_end - a.ev_begin));
       q.tiles[q.n] = tiles;
       q.first[q.n + 1] = q.first[q.n] + tiles;
       ++q.n;
@@ -2876,14 +2898,15 @@ int usx_cu_bf_execute_queue(usx_ctx* ctx, int n, usx_bf_plan* const* plans, cons
     if (q.n == 0) continue;
     q.next = next;
     USX_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream));
-    // IQ: das_csum_kernel's body (2 pixel warps x 8 channel warps); RF, and
-    // traces that body does not take: das_fast_kernel's shape.
-    auto* csum_queue = any_select ? das_csum_queue_kernel<true> : das_csum_queue_kernel<false>;
+    // IQ: das_csum_kernel's body; RF, and plans that body does not take:
+    // das_fast_kernel's shape.
+    auto* csum_queue = slim ? (any_select ? das_csum_queue_kernel<4, 4, 4, true> : das_csum_queue_kernel<4, 4, 4, false>)
+                            : (any_select ? das_csum_queue_kernel<2, 8, 8, true> : das_csum_queue_kernel<2, 8, 8, false>);
     const void* kern = cw   ? reinterpret_cast<const void*>(csum_queue)
                        : iq ? reinterpret_cast<const void*>(das_queue_kernel<true, 16, 4, 1>)
                             : reinterpret_cast<const void*>(das_queue_kernel<false, 16, 4, 1>);
     const int threads = cw ? 512 : 32 * 4;
-    const size_t tb = cw ? exp_smem_bytes(tab_events, 2, 8, 4, true) : 0;
+    const size_t tb = cw ? exp_smem_bytes(tab_events, pw, cq, 4, true) : 0;
     for (int k = 0; k < q.n; ++k) q.args[k].tab_events = tab_events;
     if (cw)
       if (int rc = smem_limit(kern, tb)) return rc;
