@@ -462,8 +462,9 @@ __global__ void __launch_bounds__(32 * kTileLines, MINB) das_fast_kernel(const B
 // values in shared memory and combines them in ascending channel order, so
 // the samples and the frames are the same bit for bit.
 //
-// What bounds it: the gathers (two 8-byte loads per pixel, channel and event:
-// L1 hit rate 50%, 42% of the L1 data pipe, 56% issue at 32 warps per SM).
+// What bounds it: the gathers' latency (two 8-byte loads per pixel, channel and
+// event; 64 x 1024 pixels, 75 events: issue 52% at 30 warps per SM, L1 38%, 4.7
+// stalls on loads and 3.5 at the passes' barriers per instruction).
 // Per frame at 128 channels, 75 plane waves, 512 x 1024 pixels:
 //   4.18 ms  the table refilled in 32-event chunks on every pass of 16
 //            channels, one channel's loads waited for before the next's
