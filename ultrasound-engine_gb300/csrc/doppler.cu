@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "usx_internal.cuh"
@@ -65,18 +66,19 @@ struct WallArgs {
 
 // The wall filter: a pixel per thread, its ensemble z[n][kWallThreads] in shared
 // memory, filtered frame i of src[j * n_pix] through the n x n projector M to
-// store(i, value), ascending i. Eight rows at a time share each read of z; M is
-// read where the kernel's arguments lie; every row sums over j in ascending
-// order, products and sums rounded separately. (in: the pixel exists. src may be
-// the frames that store writes: a thread reads its pixel whole before it writes,
-// and by ordinary loads.)
+// store(i, value), ascending i. Eight rows at a time (four, two and one of what is
+// left) share each read of z; M is read where the kernel's arguments lie; every row
+// sums over j in ascending order, products and sums rounded separately. (in: the
+// pixel exists. src may be the frames that store writes: a thread reads its pixel
+// whole before it writes, and by ordinary loads.)
 // What bounds it: latency at the occupancy that 1 KB per frame and block leaves.
-// Polynomial filter of order 2, 131,072 pixels, us, a row at a time / eight: 8
-// frames 10.4 / 10.5, 16 18.8 / 16.2, 32 43 / 42, 48 95 / 80, 64 181 / 143. With M
-// transposed in shared memory as well, for 16-byte reads of it: 17.5, 43, 140 and
-// 222 from 16 frames on (fewer blocks beside one another); 524,288 pixels, 16
-// frames, 39.6 against 47.4 here.
-constexpr int kWallThreads = 128, kWallRows = 8;
+// Polynomial filter of order 2, 131,072 pixels, us, a row at a time / this: 8
+// frames 10 / 11, 16 18.8 / 16.9, 32 43 / 39, 48 90 / 79, 56 120 / 127, 64 181 /
+// 134. M transposed in shared memory, for 16-byte reads of it, leaves fewer blocks
+// beside one another: 17.9, 44, 149, 238 and 220 from 16 frames on; only from
+// 262,144 pixels on, at 14 to 24 frames, is it the faster one (524,288 pixels, 16
+// frames, 39 against 46).
+constexpr int kWallThreads = 128;
 __host__ __device__ constexpr size_t wall_smem(int n) { return sizeof(float2) * n * kWallThreads; }
 
 template <typename Store>
@@ -91,33 +93,29 @@ __device__ __forceinline__ void wall_pixel(float4* smem, const float2* src, long
     return;
   }
   int i = 0;
-  for (; i + kWallRows <= n; i += kWallRows) {
-    float2 acc[kWallRows];
+  auto rows = [&](auto count) {   // the next count rows
+    constexpr int R = decltype(count)::value;
+    float2 acc[R];
 #pragma unroll
-    for (int r = 0; r < kWallRows; ++r) acc[r] = make_float2(0.f, 0.f);
+    for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
 #pragma unroll 2
     for (int j = 0; j < n; ++j) {
       const float2 v = z[j * kWallThreads];
 #pragma unroll
-      for (int r = 0; r < kWallRows; ++r) {
+      for (int r = 0; r < R; ++r) {
         const float m = M[(i + r) * n + j];
         acc[r].x += v.x * m;
         acc[r].y += v.y * m;
       }
     }
 #pragma unroll
-    for (int r = 0; r < kWallRows; ++r) store(i + r, acc[r]);
-  }
-  for (; i < n; ++i) {
-    float2 acc = make_float2(0.f, 0.f);
-    for (int j = 0; j < n; ++j) {
-      const float2 v = z[j * kWallThreads];
-      const float m = M[i * n + j];
-      acc.x += v.x * m;
-      acc.y += v.y * m;
-    }
-    store(i, acc);
-  }
+    for (int r = 0; r < R; ++r) store(i + r, acc[r]);
+    i += R;
+  };
+  while (i + 8 <= n) rows(std::integral_constant<int, 8>{});
+  if (i + 4 <= n) rows(std::integral_constant<int, 4>{});
+  if (i + 2 <= n) rows(std::integral_constant<int, 2>{});
+  if (i < n) rows(std::integral_constant<int, 1>{});
 }
 
 __global__ void __launch_bounds__(kWallThreads) wall_kernel(const WallArgs a) {
