@@ -314,3 +314,19 @@ def test_queues_of_few_channels_and_thin_grids(gpu):
             assert np.array_equal(o.cpu().numpy(), w)
     for p, _, _ in few + thin + full:
         p.close()
+
+
+def test_a_plane_wave_s_unused_focus_does_not_matter(gpu):
+    """Its delays are numbers: the rule's shape, and the frame."""
+    torch, capi, ctx = gpu
+    tx, channel = probe_channel(capi, 3)
+    grid = capi.Grid(0, *image_points())
+    rng = np.random.default_rng(2)
+    iq = (rng.normal(size=(3, 40, 260)) + 1j * rng.normal(size=(3, 40, 260))).astype(np.complex64)
+    want = frames_of(capi, torch, ctx, channel(), grid, iq, (0,))[0]
+    for t in tx:
+        t["focus"] = (0.0, np.nan, np.inf)
+    plan = ctx.plan(channel(), grid, capi.bf_config(f_number=1.0))
+    assert plan.variant() != 0
+    plan.close()
+    assert np.array_equal(frames_of(capi, torch, ctx, channel(), grid, iq, (None,))[0], want)

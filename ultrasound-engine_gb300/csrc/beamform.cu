@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "usx_internal.cuh"
@@ -1828,10 +1829,13 @@ bool channel_warp_samples(int n_smp) { return n_smp >= 2 && n_smp <= kMaxFastSam
 // Whether a transmit's delays are numbers at every finite point. The
 // channel-warp kernels drop an event whose sample index is not a number, where
 // das_fast_kernel's index converts to 0 and the frame shows the NaN.
-bool finite_transmit(const TxDev& t) {
-  for (float v : {t.ox, t.sin_a, t.cos_a, t.fx, t.fy, t.fz, t.axis_len, t.dx, t.dy, t.dz, t.d_origin_focus})
-    if (!std::isfinite(v)) return false;
-  return true;
+bool finite_transmit(const TxDev& t) {   // (the fields tx_arrival reads: a plane wave's focus may be at infinity)
+  auto finite = [](std::initializer_list<float> v) {
+    return std::all_of(v.begin(), v.end(), [](float x) { return std::isfinite(x); });
+  };
+  if (t.type == USX_TX_PLANE_WAVE) return finite({t.ox, t.sin_a, t.cos_a});
+  if (t.type == USX_TX_FOCUSED) return finite({t.fx, t.fy, t.fz, t.axis_len, t.dx, t.dy, t.dz});
+  return finite({t.fx, t.fy, t.fz, t.d_origin_focus});
 }
 
 // The shape of a plan whose variant was neither set nor tuned (IQ, coherent or
