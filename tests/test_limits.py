@@ -72,6 +72,28 @@ def test_demodulation_of_the_longest_traces(gpu, oracle, n_smp, taps):
     assert np.abs(iq.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("n_smp,cfg", [(30, dict(filter_taps=65)), (300, dict(filter_taps=47)),
+                                       (1100, dict(decimation=4)), (700, dict(filter_taps=127, decimation=13))])
+def test_demodulation_of_few_traces(gpu, n_smp, cfg):
+    """Blocks of one, two, four and eight traces: each trace as among nine, bit for bit."""
+    torch, capi, ctx = gpu
+    rf = torch.from_numpy(np.random.default_rng(8).standard_normal((9, n_smp)).astype(np.float32)).cuda()
+
+    def demodulated(n):
+        tx = [dict(type=1, angle=0.0, delays=np.zeros(n, np.float32), apodization=np.ones(n, np.float32))]
+        ch = capi.Channel(capi.Probe(n, 3e-4, 2.7e-4, 5e-3, 5e6, 0.6), capi.Medium(1540.0, 0.5, 1000.0),
+                          capi.Acquisition(2e7, n_smp, 1e-6, 5e3), tx)
+        iq = torch.full((n + 1, -(-n_smp // cfg.get("decimation", 1))), 7.0, dtype=torch.complex64, device="cuda")
+        ctx.demodulate(ch, capi.demod_config(**cfg), rf.data_ptr(), iq.data_ptr())
+        assert (iq[n] == 7.0).all()   # nothing past the last trace
+        return iq[:n]
+
+    want = demodulated(9)
+    assert torch.isfinite(torch.view_as_real(want)).all() and want.abs().max() > 0
+    for n in (1, 2, 3, 4, 5, 8):
+        assert torch.equal(demodulated(n), want[:n])
+
+
 def probe_channel(capi, n_ev, n_el=40, n_smp=260, kind=1, t0=0.0, iq=True):
     tx = [dict(type=kind, angle=0.1 * e - 0.1, focus=(0.0, 0.0, -0.01 - 1e-3 * e), delays=np.zeros(n_el, np.float32),
                apodization=np.ones(n_el, np.float32)) for e in range(n_ev)]
