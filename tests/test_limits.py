@@ -52,6 +52,41 @@ def test_an_element_fired_outside_the_window_adds_nothing(gpu, late):
     assert rel_l2(got, want) < 1e-6
 
 
+@pytest.mark.parametrize("full", [0, 1])
+@pytest.mark.parametrize("n_el,first", [(16, 0), (33, 32), (75, 40), (130, 65)])
+def test_records_that_end_before_the_echoes(gpu, oracle, full, n_el, first):
+    """A record of 130 samples (5 mm) of scatterers 2 to 16 mm deep, elements
+    before `first` not firing: against the oracle (FP32 sums in another order,
+    1e-5), and the samples and echo counts of a longer record's start."""
+    torch, capi, ctx = gpu
+    rng = np.random.default_rng(n_el)
+    scat = np.zeros((60, 8), np.float32)
+    scat[:, 0], scat[:, 2] = rng.uniform(-8e-3, 8e-3, 60), rng.uniform(2e-3, 0.016, 60)
+    scat[:, 3] = rng.normal(size=60)
+    z, w = np.zeros((2, n_el), np.float32), np.ones((2, n_el), np.float32)
+    w[1, :first] = 0.0
+    tx = [dict(type=1, angle=0.0, delays=z[e], apodization=w[e]) for e in range(2)]
+    cfg = dict(noise_db=-200.0, full_transmit_diffraction=full)
+    d = torch.from_numpy(scat).cuda()
+
+    def record(n_smp):
+        ch = capi.Channel(capi.Probe(n_el, 3e-4, 2.7e-4, 5e-3, 5e6, 0.6), capi.Medium(1540.0, 0.5, 1000.0),
+                          capi.Acquisition(2e7, n_smp, 0.0, 5e3), tx)
+        rf = torch.full((2, n_el, n_smp), 7.0, device="cuda")
+        count, _ = ctx.simulate(ch, capi.sim_config(**cfg), d.data_ptr(), len(scat), None, rf.data_ptr(), True)
+        return rf, count
+
+    got, count = record(130)
+    longer, more = record(600)
+    assert torch.equal(got, longer[:, :, :130]) and 0 < count < more
+    cd = O.channel_desc(O.probe(n_elements=n_el, pitch=3e-4, element_width=2.7e-4, center_frequency=5e6, bandwidth=0.6),
+                        O.medium(), O.acquisition(fs=2e7, n_samples=130, prf=5e3),
+                        O.TxSet(np.full(2, 1, np.int32), np.zeros(2, np.float32), np.zeros((2, 3), np.float32),
+                                np.zeros((2, 3), np.float32), z, w))
+    want = oracle.simulate(cd, O.sim_config(**cfg), scat)
+    assert np.abs(want).max() > 0 and rel_l2(got.cpu().numpy(), want) < 1e-5
+
+
 @pytest.mark.parametrize("n_smp,taps", [(14679840, 33), (14680064, 33), (14680064, 21)])
 def test_demodulation_of_the_longest_traces(gpu, oracle, n_smp, taps):
     """65,535 segments of 224 outputs, and one more: against the oracle, tap by
